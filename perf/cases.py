@@ -299,3 +299,73 @@ def tolerance(case):
             "linear": {"rel": 0.003, "max": 0.016},
             "head": {"rel": 0.007, "max": 0.03},
             "moe": {"rel": 0.01, "max": 0.08}}[case["kind"]]
+
+
+# --------------------------------------------------------------------------- the same in 64 bits
+def _exact_attention(case, s):
+    """Sequence by sequence, KV head by KV head, 1024 queries at a time."""
+    ql, kl = _lengths(case)
+    h, hk, causal = case["heads"], case["kv_heads"], case["causal"]
+    g, scale = h // hk, 1.0 / math.sqrt(D)
+    f = dict(dtype=torch.float64, device=DEV)
+    out, dq = torch.zeros(sum(ql), h, D, **f), torch.zeros(sum(ql), h, D, **f)
+    dk, dv = torch.zeros(sum(kl), hk, D, **f), torch.zeros(sum(kl), hk, D, **f)
+    lse = torch.full((len(ql), h, max(ql)), float("-inf"), **f)
+    q0 = k0 = 0
+    for i, (nq, nk) in enumerate(zip(ql, kl)):
+        for c in range(hk):
+            k, v = s["k"][k0:k0 + nk, c].double(), s["v"][k0:k0 + nk, c].double()
+            for a in range(0, nq, 1024):
+                n = min(1024, nq - a)
+                rows, hs = slice(q0 + a, q0 + a + n), slice(c * g, (c + 1) * g)
+                q = s["q"][rows, hs].double().transpose(0, 1).reshape(g * n, D)
+                do = s["dout"][rows, hs].double().transpose(0, 1).reshape(g * n, D)
+                p = q @ k.t() * scale
+                if causal:
+                    last = torch.arange(a, a + n, device=DEV).repeat(g)[:, None] + (nk - nq)
+                    p.masked_fill_(torch.arange(nk, device=DEV)[None] > last, float("-inf"))
+                l = torch.logsumexp(p, dim=1, keepdim=True)
+                p = torch.exp(p - l)
+                o = p @ v
+                ds = p * (do @ v.t() - (do * o).sum(1, keepdim=True)) * scale
+                out[rows, hs] = o.view(g, n, D).transpose(0, 1)
+                dq[rows, hs] = (ds @ k).view(g, n, D).transpose(0, 1)
+                dk[k0:k0 + nk, c] += ds.t() @ q
+                dv[k0:k0 + nk, c] += p.t() @ do
+                lse[i, hs, a:a + n] = l.view(g, n)
+        q0, k0 = q0 + nq, k0 + nk
+    return dict(out=out, lse=None if min(ql) < max(ql) else lse, dq=dq, dk=dk, dv=dv)
+
+
+def _exact_head(case, s):
+    """512 tokens at a time; the loss with label smoothing as ``dhellam_b200/ops/loss.py`` states it."""
+    t, v = case["tokens"], case["vocab"]
+    smooth = case["label_smoothing"] * v / (v - 1)
+    w = s["w"].double()
+    loss, dlogits, dx, dw = [], [], [], torch.zeros_like(w)
+    for a in range(0, t, 512):
+        x, labels = s["x"][a:a + 512].double(), s["labels"][a:a + 512, None]
+        logits = x @ w.t()
+        lse = torch.logsumexp(logits, dim=1, keepdim=True)
+        loss.append(((1 - smooth) * (lse - logits.gather(1, labels)) - smooth * (logits.mean(1, keepdim=True) - lse)).squeeze(1))
+        d = torch.exp(logits - lse) - smooth / v
+        d.scatter_add_(1, labels, torch.full_like(d[:, :1], smooth - 1))
+        d *= s["dloss"][a:a + 512, None].double()
+        dlogits.append(d.float())
+        dx.append(d @ w)
+        dw += d.t() @ x
+    return dict(loss=torch.cat(loss), dlogits=torch.cat(dlogits), dx=torch.cat(dx), dw=dw)
+
+
+def exact(case, seed):
+    """No value for a training step (every layer rounds to bf16 what the next one reads) nor for the experts (tokens whose
+    routes are nearly tied go elsewhere in 64 bits)."""
+    if case["kind"] not in ("attention", "linear", "head"):
+        return None
+    s = prepare(case, seed)
+    if case["kind"] == "attention":
+        return _exact_attention(case, s)
+    if case["kind"] == "head":
+        return _exact_head(case, s)
+    x, w, dy = s["x"].double(), s["w"].double(), s["dy"].double()
+    return dict(y=x @ w.t(), dx=dy @ w, dw=dy.t() @ x)
