@@ -1,30 +1,49 @@
 // Flash attention forward and backward for sm_100a (head size 128, bf16, grouped KV heads,
-// causal or full, strided [S, B, heads, d] operands so a packed QKV buffer needs no copies).
+// causal or full, strided [S, B, heads, d] operands so a packed QKV buffer needs no copies;
+// packed batches of sequences of unequal length in one launch).
 //
-// Forward, one CTA per (128 query rows, batch, query head):
-//   warp 0     TMA producer: Q once, then K_j / V_j tiles through 2-stage rings
-//   warp 1     MMA issuer:   S_j = Q K_j^T and O_j = P_j V_j with tcgen05.mma, S and O tiles
-//                            double-buffered in TMEM (4 x 128 columns = all 512)
-//   warps 2-9  softmax:      two warps per TMEM lane quarter; both own the same 32 query rows, each
-//                            takes 64 of the 128 score columns and 64 of the 128 output columns: two
-//                            passes over its part of S_j in TMEM (row max, exchanged inside the pair
-//                            through shared memory; then exp2 / row sum / bf16 P_j into swizzled
-//                            shared memory), running output kept in registers (64 per thread) and
-//                            rescaled once per block
-//   S_{j+1} and P_{j-1} V_{j-1} run on the tensor cores while the softmax warps work on S_j.
+// What bounds it: per pair of 128-row tiles the tensor cores need 512 cycles per product (two
+// forward, seven backward) and the 128 x 128 exponentials 1024 cycles of the special-function
+// units, so the kernels are built to keep both busy at once:
+//
+// Forward, one CTA per two tiles of 128 query rows that share their keys (two query heads of a
+// KV group; for groups of odd size two neighbouring row tiles of one head):
+//   warp 0      TMA producer: Q tiles once, then K_j / V_j through one 5-slot ring
+//   warp 1      MMA issuer:   S_t = Q_t K_j^T, O_t += P_t V_j (t = 0, 1) with P read from TMEM
+//   warps 4-7, 8-11  softmax of tile 0 / 1: one thread per row, no exchange between threads; P_t
+//               overwrites S_t in TMEM as bf16; O_t stays in TMEM and is rescaled only when a
+//               row's maximum has grown by more than 2^8 (any reference maximum gives the same
+//               quotient; a stale one only scales numerator and denominator)
+//   While one tile is in softmax the tensor cores work on the other.
+//   Measured, causal, 8 query heads on 2 KV heads: 32768 positions 3628 us -> 1850 us, 16384 positions 452 us (1.22 PFLOP/s);
+//   tensor and special-function pipes each ~66 % busy, the rest is the chain softmax -> P V -> S of one tile (two softmax
+//   warps per scheduler).  Tried and slower: steps of 64 keys with S double-buffered (an N = 64 product takes as long as an
+//   N = 128 one: 2116 against 1550 cycles per tile pair); 1/8 to 1/2 of the exponentials as a polynomial on the FMA pipe
+//   (4 to 20 % slower: the warps are bound by instruction latency, not by the special-function pipe).
 //
 // Backward is two kernels that share delta = rowsum(dO * O):
 //   dK/dV: one CTA per (128 keys, batch, KV head) loops over the query heads of the group and
-//     the query blocks that see these keys: S = Q K^T and dP = dO V^T into TMEM; eight math
-//     warps form P = exp2(S - lse) and dS = P (dP - delta) into swizzled shared-memory images
-//     that are consumed as MN-major operands (dV += P^T dO, dK += dS^T Q), so no transposed
-//     copies exist anywhere; dK / dV accumulate in TMEM over the whole loop, which also sums
-//     the query heads of a KV group.  When keys x batch x KV heads gives too few CTAs for the
-//     machine (one KV head per GPU under tensor parallelism), the query heads of a group are
-//     split over up to 8 CTAs that write fp32 partials, and attn_dkv_reduce_kernel adds them.
+//     the query blocks that see these keys.  Scores are formed transposed (keys on TMEM lanes),
+//     so P^T = exp2(S^T - lse) and dS^T = P^T (dP^T - delta) go back to TMEM as they stand and are
+//     the A operands of dV += P^T dO and dK += dS^T Q: no shared-memory round trip, and the MMAs
+//     read half the shared memory.  The math warps' P phase runs beside dK(i-1), dP(i) and the dS
+//     phase beside dV(i), S(i+1), so nothing is double-buffered in TMEM.  When keys x batch x KV
+//     heads gives too few CTAs (one KV head per GPU under tensor parallelism), the query heads
+//     of a group are split over up to 8 CTAs that write fp32 partials; attn_dkv_reduce_kernel
+//     adds them in a fixed order.
 //   dQ: one CTA per (128 queries, batch, query head) loops over the key blocks, recomputes S
-//     and dP and accumulates dQ += dS K in TMEM.  Recomputing two products per tile pair
-//     replaces an fp32 atomic accumulation of dQ, which was bound by L2 atomic throughput.
+//     and dP and accumulates dQ += dS K in TMEM (dS again as a TMEM operand).  Recomputing two
+//     products per tile pair replaces an fp32 atomic accumulation of dQ and keeps dQ reproducible.
+//   Measured (same shape, 32768): dK/dV 7833 us -> 3520 us, dQ 5326 us -> 2250 us.  The forms before ran one phase after
+//   the other and applied the mask as predicates (10 ALU instructions per score in dQ).
+//
+// MMAs are issued under a predicate by a warp whose control flow stays uniform (ptx.cuh, umma_bf16_by): issued inside
+// `if (lane == 0)` a 128 x 128 x 16 product took 75-100 cycles to issue, against 64 to execute.
+//
+// Packed batches: the row offsets of the sequences and a list of (sequence, tile) in descending
+// order of work travel as a kernel parameter; tiles are cut by the sequence's own length, and rows
+// of the next sequence that a tile load brings in are zeroed where they enter a contraction (zero
+// probability times a neighbour's NaN would be NaN).
 //
 // Role in the reference: the bundled flash-attention 2 sm80 kernels behind
 // pymha_varlen_fwd / pymha_varlen_bwd (csrc/operators/flash_atten.cu:220-434, 479-757);
@@ -35,8 +54,11 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
+#include <vector>
 
 #include "api.h"
 #include "ptx.cuh"
@@ -48,17 +70,61 @@ namespace attn {
 constexpr int BQ = 128, BKV = 128, D = 128;
 constexpr int HALF_BYTES = 128 * 128;        // one [128 rows][64 elems] swizzled box
 constexpr int TILE_BYTES = 2 * HALF_BYTES;   // [128][128] bf16
-constexpr int THREADS = 192;
-constexpr int BWD_THREADS = 320;           // TMA warp + MMA warp + 8 math warps (two per TMEM lane quarter)
+constexpr int THREADS = 384;                 // warp 0 TMA, warp 1 MMA, warps 2-3 helpers, warps 4-11 math
+constexpr int MATH_WARP0 = 4;
 constexpr float LOG2E = 1.4426950408889634f;
 
-struct Geometry {
-  int B, Hq, Hk, Sq, Sk, causal;
-  float scale;
-  long long o_s, o_b, o_h;        // output strides (elements)
-  DeviceStatus* status;
-  int x0, p0, ny;                 // SM budget: this launch covers tile columns from x0 and (head, batch) pairs from p0; ny = heads
+// Sequences and tiles of one packed launch (a kernel parameter: no device table, nothing to copy or keep).
+constexpr int MAX_SEQS = 128, MAX_TILES = 768;
+struct Packed {
+  int q0[MAX_SEQS], k0[MAX_SEQS];            // first row in the packed tensors
+  int nq[MAX_SEQS], nk[MAX_SEQS];            // rows
+  int id[MAX_SEQS];                          // position in the batch (row of the statistics)
+  uint32_t tile[MAX_TILES];                  // sequence << 16 | tile
 };
+struct Dense {};                             // equal lengths: everything follows from the block index
+
+struct Geometry {
+  int B, Hq, Hk;                             // batch dimension of the tensors (1 when packed)
+  int Sq, Sk;                                // rows per sequence (dense only)
+  int Tq, Tk;                                // rows of the tensors' sequence dimension
+  int ls;                                    // row stride of the statistics [.., Hq, ls]
+  int causal;
+  float scale;
+  int x0;                                    // first work item of this launch (SM budget: launches in waves)
+  int heads;                                 // work items per tile and batch entry
+  DeviceStatus* status;
+};
+
+// One tile's surroundings: sequence bounds and where its rows start.
+struct Work {
+  int b, head, tile, sid;                    // batch coordinate, head item, tile, row of the statistics
+  int q0, k0, nq, nk;
+};
+
+// Heaviest tiles first over ALL heads and sequences: the tile index is the slowest part of the work item.
+template <class Table>
+__device__ __forceinline__ Work find_work(const Geometry& g, const Table& t, int item) {
+  Work w;
+  if constexpr (sizeof(Table) > 1) {
+    w.head = item % g.heads;
+    const uint32_t e = t.tile[item / g.heads];
+    const int s = (int)(e >> 16);
+    w.tile = (int)(e & 0xffffu);
+    w.b = 0;
+    w.sid = t.id[s];
+    w.q0 = t.q0[s]; w.k0 = t.k0[s]; w.nq = t.nq[s]; w.nk = t.nk[s];
+  } else {
+    const int per = g.heads * g.B;
+    const int i = item % per;
+    w.tile = item / per;
+    w.head = i % g.heads;
+    w.b = i / g.heads;
+    w.sid = w.b;
+    w.q0 = 0; w.k0 = 0; w.nq = g.Sq; w.nk = g.Sk;
+  }
+  return w;
+}
 
 // K-major operand descriptor for step kk (16 elements of the contraction) of a tile stored
 // as two [128][64] swizzled boxes.
@@ -69,54 +135,114 @@ __device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int kk) {
 __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int kk) {
   return umma_smem_desc(base + kk * 2048, HALF_BYTES, 1024);
 }
-// Byte offset of 16-byte chunk c (0..15) of row r in the two-box swizzled image.
-__device__ __forceinline__ uint32_t swz_off(int r, int c) {
-  return (uint32_t)((c >> 3) * HALF_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int head, int b, int row) {
+  tma_load_4d(dst, m, bar, 0, head, b, row);
+  tma_load_4d(dst + HALF_BYTES, m, bar, 64, head, b, row);
+}
+// Bounded wait of a whole warp with one answer for all lanes, so that the control flow behind it stays uniform.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, DeviceStatus* st, int where) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, st, where));
+}
+// Zeroes rows [first, 128) of a tile in shared memory (whole warp); a row is 128 bytes in each of the two boxes.
+__device__ __forceinline__ void zero_tile_rows(uint8_t* tile, int first, int lane) {
+  for (int h = 0; h < 2; ++h)
+    for (int o = first * 128 + lane * 16; o < HALF_BYTES; o += 512) *reinterpret_cast<uint4*>(tile + h * HALF_BYTES + o) = make_uint4(0, 0, 0, 0);
+  fence_proxy_async_smem();
+  __syncwarp();
+}
+
+// ---- packed fp32 arithmetic: two lanes per instruction, same rounding as the scalar forms
+__device__ __forceinline__ uint64_t pk2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Key j of the tile is visible to a row iff j < limit.
+__device__ __forceinline__ int visible_keys(int nk, int causal, int off, int qi, int key0) {
+  int limit = nk - key0;
+  if (causal) limit = min(limit, qi + off - key0 + 1);
+  return limit;
 }
 
 // ======================================================================= forward
+constexpr int FWD_RING = 5;
 struct FwdCtl {
-  uint64_t q_full;
-  uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
-  uint64_t s_full[2], p_ready[2], o_full[2];
+  uint64_t q_full[2];
+  uint64_t kv_full[FWD_RING], kv_empty[FWD_RING];
+  uint64_t s_full[2], p_ready[2][2], o_done[2];   // [tile], p_ready [tile][half of the keys]
   uint32_t tmem_base;
   int abort_flag;
-  float xch[2 * 128];            // row maximum / row sum exchange between the two softmax warps of a row
 };
-constexpr int FWD_THREADS = 320;                         // TMA warp + MMA warp + 8 softmax warps
-constexpr int FWD_SMEM = TILE_BYTES * 7 + 1024 + 1280;  // Q, K x2, V x2, P x2, control
+constexpr int FWD_SMEM = TILE_BYTES * (2 + FWD_RING) + 1024 + 512;
+constexpr float RESCALE_LOG2 = 8.f;          // P stays below 2^8: as exact in bf16 as below 1
 
-__global__ void __launch_bounds__(FWD_THREADS, 1)
+struct FwdArgs {
+  __nv_bfloat16* out;
+  float* lse;
+  long long o_s, o_b, o_h;                   // output strides (elements)
+  int head_pair;                             // 1: a CTA's two tiles are query heads 2h, 2h+1; 0: row tiles 2i, 2i+1 of one head
+};
+
+template <class Table>
+__global__ void __launch_bounds__(THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                __nv_bfloat16* __restrict__ out, float* __restrict__ lse, const Geometry g) {
+                const __grid_constant__ Geometry g, const __grid_constant__ FwdArgs a, const __grid_constant__ Table table) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sK = smem + TILE_BYTES;
-  uint8_t* sV = smem + 3 * TILE_BYTES;
-  uint8_t* sP = smem + 5 * TILE_BYTES;
-  FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + 7 * TILE_BYTES);
+  uint8_t* sKV = smem + 2 * TILE_BYTES;
+  FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + (2 + FWD_RING) * TILE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqb = (g.Sq + BQ - 1) / BQ;
-  const int qb = nqb - 1 - (g.x0 + (int)blockIdx.x);       // heaviest (latest) query blocks first
-  const int pyz = g.p0 + (int)blockIdx.y + (int)blockIdx.z * (int)gridDim.y;
-  const int hq = pyz % g.ny, b = pyz / g.ny;
-  const int hk = hq / (g.Hq / g.Hk);
-  const int off = g.Sk - g.Sq;                    // key j visible to query i iff j <= i + off
-  int nblk = (g.Sk + BKV - 1) / BKV;
-  if (g.causal) {
-    const int last_key = qb * BQ + BQ - 1 + off;
-    nblk = last_key < 0 ? 0 : min(nblk, last_key / BKV + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const Work w = find_work(g, table, g.x0 + (int)blockIdx.x);
+  const int off = w.nk - w.nq;                     // key j visible to query i iff j <= i + off
+  const int hq_[2] = {a.head_pair ? 2 * w.head : w.head, a.head_pair ? 2 * w.head + 1 : w.head};
+  const int hk = hq_[0] / (g.Hq / g.Hk);
+  // dense tiles are counted from the end: the latest queries see most keys
+  const int per_cta = a.head_pair ? BQ : 2 * BQ;
+  const int last = (w.nq + per_cta - 1) / per_cta - 1;
+  const int tile = sizeof(Table) > 1 ? w.tile : last - w.tile;
+  const int qb_[2] = {a.head_pair ? tile : 2 * tile, a.head_pair ? tile : 2 * tile + 1};
+  int nblk_[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    int n = (w.nk + BKV - 1) / BKV;
+    if (g.causal) {
+      const int last_key = min(qb_[t] * BQ + BQ, w.nq) - 1 + off;
+      n = last_key < 0 ? 0 : min(n, last_key / BKV + 1);
+    }
+    nblk_[t] = qb_[t] * BQ < w.nq ? n : 0;
   }
+  const int nmax = max(nblk_[0], nblk_[1]);
 
   if (threadIdx.x == 0) {
-    mbar_init(&ctl->q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&ctl->k_full[i], 1); mbar_init(&ctl->k_empty[i], 1);
-      mbar_init(&ctl->v_full[i], 1); mbar_init(&ctl->v_empty[i], 1);
-      mbar_init(&ctl->s_full[i], 1); mbar_init(&ctl->p_ready[i], 8); mbar_init(&ctl->o_full[i], 1);
+      mbar_init(&ctl->q_full[i], 1);
+      mbar_init(&ctl->s_full[i], 1); mbar_init(&ctl->p_ready[i][0], 4); mbar_init(&ctl->p_ready[i][1], 4); mbar_init(&ctl->o_done[i], 1);
     }
+    for (int i = 0; i < FWD_RING; ++i) { mbar_init(&ctl->kv_full[i], 1); mbar_init(&ctl->kv_empty[i], 1); }
     ctl->abort_flag = 0;
     mbar_fence_init();
   }
@@ -124,202 +250,197 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort_flag;
+  // TMEM columns: S_0 [0,128) S_1 [128,256), each overwritten by its bf16 P in the first 64; O_0 [256,384) O_1 [384,512)
 
   if (warp == 0) {
-    if (lane == 0 && nblk > 0) {
+    if (lane == 0 && nmax > 0) {
       tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
-      mbar_expect_tx(&ctl->q_full, TILE_BYTES);
-      tma_load_4d(sQ, &tq, &ctl->q_full, 0, hq, b, qb * BQ);
-      tma_load_4d(sQ + HALF_BYTES, &tq, &ctl->q_full, 64, hq, b, qb * BQ);
-      for (int j = 0; j < nblk; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&ctl->k_empty[s], ph ^ 1, abort_flag, g.status, 400)) break;
-        mbar_expect_tx(&ctl->k_full[s], TILE_BYTES);
-        tma_load_4d(sK + s * TILE_BYTES, &tk, &ctl->k_full[s], 0, hk, b, j * BKV);
-        tma_load_4d(sK + s * TILE_BYTES + HALF_BYTES, &tk, &ctl->k_full[s], 64, hk, b, j * BKV);
-        if (!mbar_wait(&ctl->v_empty[s], ph ^ 1, abort_flag, g.status, 401)) break;
-        mbar_expect_tx(&ctl->v_full[s], TILE_BYTES);
-        tma_load_4d(sV + s * TILE_BYTES, &tv, &ctl->v_full[s], 0, hk, b, j * BKV);
-        tma_load_4d(sV + s * TILE_BYTES + HALF_BYTES, &tv, &ctl->v_full[s], 64, hk, b, j * BKV);
+      int slot = 0;
+      uint32_t ph = 1;
+      for (int i = 0; i < 2 * nmax; ++i) {          // K_0 V_0 K_1 V_1 ...
+        if (i < 2 && nblk_[i] > 0) {                // Q_0 goes before K_0, Q_1 before V_0
+          mbar_expect_tx(&ctl->q_full[i], TILE_BYTES);
+          load_tile(sQ + i * TILE_BYTES, &tq, &ctl->q_full[i], hq_[i], w.b, w.q0 + qb_[i] * BQ);
+        }
+        if (!mbar_wait(&ctl->kv_empty[slot], ph, abort_flag, g.status, 400)) break;
+        mbar_expect_tx(&ctl->kv_full[slot], TILE_BYTES);
+        load_tile(sKV + slot * TILE_BYTES, (i & 1) ? &tv : &tk, &ctl->kv_full[slot], hk, w.b, w.k0 + (i >> 1) * BKV);
+        if (++slot == FWD_RING) { slot = 0; ph ^= 1; }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && nblk > 0) {
+    const uint32_t leader = elect_one();
+    if (nmax > 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, 0, 1);
-      const uint32_t q_base = smem_u32(sQ);
-      bool ok = mbar_wait(&ctl->q_full, 0, abort_flag, g.status, 410);
-      auto issue_s = [&](int j) -> bool {
-        const int s = j & 1;
-        if (!mbar_wait(&ctl->k_full[s], (j >> 1) & 1, abort_flag, g.status, 411)) return false;
+      // load i of the ring (K of block j: 2 j, V: 2 j + 1)
+      auto wait_load = [&](int i, int where) {
+        const bool r = warp_wait(&ctl->kv_full[i % FWD_RING], (i / FWD_RING) & 1, abort_flag, g.status, where);
         tc_fence_after();
-        const uint32_t k_base = smem_u32(sK + s * TILE_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + s * 128, desc_kmajor(q_base, kk), desc_kmajor(k_base, kk), idesc_s, kk > 0);
-        umma_commit(&ctl->k_empty[s]);
-        umma_commit(&ctl->s_full[s]);
-        return true;
+        return r;
       };
-      if (ok) ok = issue_s(0);
-      if (ok && nblk > 1) ok = issue_s(1);
-      for (int j = 0; j < nblk && ok; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&ctl->p_ready[s], ph, abort_flag, g.status, 412)) break;
-        if (!mbar_wait(&ctl->v_full[s], ph, abort_flag, g.status, 413)) break;
-        tc_fence_after();
-        const uint32_t p_base = smem_u32(sP + s * TILE_BYTES);
-        const uint32_t v_base = smem_u32(sV + s * TILE_BYTES);
+      auto issue_s = [&](int t, int j) {
+        const uint32_t q_base = smem_u32(sQ + t * TILE_BYTES), k_base = smem_u32(sKV + (2 * j % FWD_RING) * TILE_BYTES);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 256 + s * 128, desc_kmajor(p_base, kk), desc_mnmajor(v_base, kk), idesc_pv, kk > 0);
-        umma_commit(&ctl->v_empty[s]);
-        umma_commit(&ctl->o_full[s]);
-        if (j + 2 < nblk) ok = issue_s(j + 2);
+        for (int kk = 0; kk < 8; ++kk) umma_bf16_by(leader, tmem + t * 128, desc_kmajor(q_base, kk), desc_kmajor(k_base, kk), idesc_s, kk > 0);
+        umma_commit_by(leader, &ctl->s_full[t]);
+      };
+      bool ok = wait_load(0, 410);
+      for (int t = 0; t < 2 && ok; ++t) {
+        if (nblk_[t] == 0) continue;
+        ok = warp_wait(&ctl->q_full[t], 0, abort_flag, g.status, 411);
+        tc_fence_after();
+        if (ok) issue_s(t, 0);
+      }
+      umma_commit_by(leader, &ctl->kv_empty[0]);
+      for (int j = 0; j < nmax && ok; ++j) {
+        uint8_t* vtile = sKV + ((2 * j + 1) % FWD_RING) * TILE_BYTES;
+        if (!wait_load(2 * j + 1, 412)) { ok = false; break; }
+        if (sizeof(Table) > 1 && (j + 1) * BKV > w.nk && w.k0 + w.nk < g.Tk) zero_tile_rows(vtile, w.nk - j * BKV, lane);
+        const uint32_t v_base = smem_u32(vtile);
+        bool have_k = false;
+        for (int t = 0; t < 2 && ok; ++t) {
+          if (j >= nblk_[t]) continue;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {              // the first half of P V runs beside the exponentials of the second
+            if (!warp_wait(&ctl->p_ready[t][h], j & 1, abort_flag, g.status, 413)) ok = false;
+            tc_fence_after();
+            if (ok) {
+#pragma unroll
+              for (int kk = 4 * h; kk < 4 * h + 4; ++kk)
+                umma_bf16_ts_by(leader, tmem + 256 + t * 128, tmem + t * 128 + kk * 8, desc_mnmajor(v_base, kk), idesc_pv, (j | kk) != 0);
+            }
+          }
+          if (!ok) break;
+          if (j + 1 < nblk_[t]) {
+            if (!have_k && !wait_load(2 * j + 2, 414)) { ok = false; break; }
+            have_k = true;
+            issue_s(t, j + 1);                       // in order behind the P V that reads the same columns
+          } else {
+            umma_commit_by(leader, &ctl->o_done[t]);
+          }
+        }
+        if (!ok) break;
+        umma_commit_by(leader, &ctl->kv_empty[(2 * j + 1) % FWD_RING]);
+        if (have_k) umma_commit_by(leader, &ctl->kv_empty[(2 * j + 2) % FWD_RING]);
       }
     }
     __syncwarp();
-  } else {
-    // Eight softmax warps: two per TMEM lane quarter.  Both warps of a pair own the same 32 query rows;
-    // warp half `hf` handles score columns [64 hf, 64 hf + 64) of every key block and head-dim columns
-    // [64 hf, 64 hf + 64) of the running output.  The row maximum is exchanged through shared memory
-    // (one named barrier per pair), the row sums are added once at the end.  Two warps per scheduler hide
-    // the TMEM round trips that a single warp per scheduler exposes.  A warp whose wait gives up keeps
-    // walking the loop (every later wait returns at once through the CTA's abort flag), so the pair's
-    // barriers always match.
+  } else if (warp >= MATH_WARP0) {
+    const int t = (warp - MATH_WARP0) >> 2;
     const int quarter = warp & 3;
-    const int hf = (warp - 2) >> 2;
-    const int r = quarter * 32 + lane;               // row inside the tile
-    const int qi = qb * BQ + r;                      // global query index
+    const int qi = qb_[t] * BQ + quarter * 32 + lane;
+    const bool row_ok = qi < w.nq;
+    const int nblk = nblk_[t];
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t ts = tmem + t * 128 + lane_base, to = tmem + 256 + t * 128 + lane_base;
     const float sl2 = g.scale * LOG2E;
-    float* xch = ctl->xch;                           // [2][128] exchange between the two warps of a pair
-    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); };
-    float m = -FLT_MAX, l = 0.f;
-    float o[64];
-#pragma unroll
-    for (int i = 0; i < 64; ++i) o[i] = 0.f;
+    const uint64_t sl2_2 = pk2(sl2, sl2);
+    float m = -INFINITY;                             // reference maximum of the row (raw score)
+    uint64_t l2 = pk2(0.f, 0.f);                     // row sum in two interleaved parts
     bool ok = nblk > 0;
-    for (int j = 0; j < nblk; ++j) {
-      const int s = j & 1;
-      const uint32_t ph = (j >> 1) & 1;
-      if (ok && !mbar_wait(&ctl->s_full[s], ph, abort_flag, g.status, 420)) ok = false;
+    for (int j = 0; j < nblk && ok; ++j) {
+      if (!mbar_wait(&ctl->s_full[t], j & 1, abort_flag, g.status, 420)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t ts = tmem + s * 128 + lane_base + hf * 64;
-      const int key0 = j * BKV + hf * 64;            // first key of this warp's columns
-      int limit = g.Sk - key0;                                        // keys beyond Sk are padding
-      if (g.causal) limit = min(limit, qi + off - key0 + 1);
-      const bool full_block = limit >= 64;
-      // pass 1: row maximum over this warp's 64 columns, then over the pair
-      float bm = -FLT_MAX;
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
-        uint32_t v[32];
-        tmem_ld32(ts + c * 32, v);
-        tmem_ld_wait();
-        if (full_block) {
+      const int limit = visible_keys(w.nk, g.causal, off, qi, j * BKV);
+      const bool full = __all_sync(0xffffffffu, limit >= BKV);
+      uint32_t s[BKV];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) bm = fmaxf(bm, __uint_as_float(v[i]));
-        } else {
+      for (int c = 0; c < 4; ++c) tmem_ld32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
+      tmem_ld_wait();
+      if (!full) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) if (c * 32 + i < limit) bm = fmaxf(bm, __uint_as_float(v[i]));
-        }
+        for (int i = 0; i < BKV; ++i) if (i >= limit) s[i] = __float_as_uint(-INFINITY);
       }
-      xch[hf * 128 + r] = bm;
-      pair_sync();
-      bm = fmaxf(bm, xch[(hf ^ 1) * 128 + r]);
-      pair_sync();                                   // the partner has read before the next block overwrites
-      const float m_new = fmaxf(m, bm);
-      const float alpha = (m == -FLT_MAX) ? 0.f : exp2f((m - m_new) * sl2);
-      const float mb = (m_new == -FLT_MAX) ? 0.f : m_new * sl2;
-      // pass 2: probabilities -> shared memory (bf16, swizzled), partial row sum
-      float rs = 0.f;
-      uint8_t* pdst = sP + s * TILE_BYTES;
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
-        uint32_t v[32];
-        tmem_ld32(ts + c * 32, v);
-        tmem_ld_wait();
-        float p[32];
+      float mx[4];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float e = exp2f(__uint_as_float(v[i]) * sl2 - mb);
-          if (!full_block && c * 32 + i >= limit) e = 0.f;
-          p[i] = e;
-          rs += e;
-        }
+      for (int c = 0; c < 4; ++c) mx[c] = __uint_as_float(s[c]);
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint4 u;
-          u.x = pack_bf16x2(p[q4 * 8 + 0], p[q4 * 8 + 1]);
-          u.y = pack_bf16x2(p[q4 * 8 + 2], p[q4 * 8 + 3]);
-          u.z = pack_bf16x2(p[q4 * 8 + 4], p[q4 * 8 + 5]);
-          u.w = pack_bf16x2(p[q4 * 8 + 6], p[q4 * 8 + 7]);
-          *reinterpret_cast<uint4*>(pdst + swz_off(r, hf * 8 + c * 4 + q4)) = u;
-        }
+      for (int i = 4; i < BKV; i += 4) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mx[c] = fmaxf(mx[c], __uint_as_float(s[i + c]));
       }
-      l = l * alpha + rs;
-      m = m_new;
-      tc_fence_before();
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->p_ready[s]);
-      // fold in the previous block's P V (relative to the previous maximum), then rescale: this warp's 64 head-dim columns
-      if (j > 0) {
-        const int sp = (j - 1) & 1;
-        if (ok && !mbar_wait(&ctl->o_full[sp], ((j - 1) >> 1) & 1, abort_flag, g.status, 421)) ok = false;
-        tc_fence_after();
-        const uint32_t to = tmem + 256 + sp * 128 + lane_base + hf * 64;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t v[32];
-          tmem_ld32(to + c * 32, v);
+      const float bm = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      if (j == 0) {
+        m = bm;
+      } else if (__any_sync(0xffffffffu, (bm - m) * sl2 > RESCALE_LOG2)) {
+        // a reference of -inf (nothing seen yet) has zero sums: any factor will do, 0 is finite
+        const float m_new = fmaxf(m, bm);
+        const float alpha = m == -INFINITY ? 0.f : ex2((m - m_new) * sl2);
+        m = m_new;
+        l2 = mul2(l2, pk2(alpha, alpha));
+        // S_t(j) was issued behind P V of block j - 1, so O_t is complete up to that block
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {
+          uint32_t o[16];
+          tmem_ld16(to + c * 16, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[c * 32 + i] = (o[c * 32 + i] + __uint_as_float(v[i])) * alpha;
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st16(to + c * 16, o);
         }
+      }
+      const float nm = m == -INFINITY ? 0.f : -m * sl2;
+      const uint64_t nm2 = pk2(nm, nm);
+      uint64_t rs[2] = {0, 0};                       // the block's own sum: short chains, then one add to the running sum
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int c = 4 * h; c < 4 * h + 4; ++c) {
+          uint32_t p[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int e = c * 16 + 2 * i;
+            float x, y;
+            upk2(fma2(pk2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sl2_2, nm2), x, y);
+            x = ex2(x); y = ex2(y);
+            rs[i & 1] = add2(rs[i & 1], pk2(x, y));
+            p[i] = pack_bf16x2(x, y);
+          }
+          tmem_st8(ts + c * 8, p);
+        }
+        tmem_st_wait();
         tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->p_ready[t][h]);
       }
+      l2 = add2(l2, add2(rs[0], rs[1]));
     }
-    // the row sum of the whole row = the two halves' partial sums (same running maximum in both)
-    xch[hf * 128 + r] = l;
-    pair_sync();
-    l += xch[(hf ^ 1) * 128 + r];
+    float l0, l1;
+    upk2(l2, l0, l1);
+    const float l = l0 + l1;
+    __nv_bfloat16* orow = a.out + (long long)(w.q0 + qi) * a.o_s + (long long)w.b * a.o_b + (long long)hq_[t] * a.o_h;
+    float* lrow = a.lse + ((long long)w.sid * g.Hq + hq_[t]) * g.ls + qi;
     if (nblk > 0) {
-      const int sp = (nblk - 1) & 1;
-      if (ok && !mbar_wait(&ctl->o_full[sp], ((nblk - 1) >> 1) & 1, abort_flag, g.status, 422)) ok = false;
-      if (ok) {
+      if (ok && mbar_wait(&ctl->o_done[t], 0, abort_flag, g.status, 422)) {
         tc_fence_after();
-        const uint32_t to = tmem + 256 + sp * 128 + lane_base + hf * 64;
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        __nv_bfloat16* orow = out + (long long)qi * g.o_s + (long long)b * g.o_b + (long long)hq * g.o_h + hf * 64;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < 4; ++c) {
           uint32_t v[32];
           tmem_ld32(to + c * 32, v);
           tmem_ld_wait();
-          if (qi < g.Sq) {
+          if (row_ok) {
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
               uint4 u;
               const int i0 = q4 * 8;
-              u.x = pack_bf16x2((o[c * 32 + i0 + 0] + __uint_as_float(v[i0 + 0])) * inv, (o[c * 32 + i0 + 1] + __uint_as_float(v[i0 + 1])) * inv);
-              u.y = pack_bf16x2((o[c * 32 + i0 + 2] + __uint_as_float(v[i0 + 2])) * inv, (o[c * 32 + i0 + 3] + __uint_as_float(v[i0 + 3])) * inv);
-              u.z = pack_bf16x2((o[c * 32 + i0 + 4] + __uint_as_float(v[i0 + 4])) * inv, (o[c * 32 + i0 + 5] + __uint_as_float(v[i0 + 5])) * inv);
-              u.w = pack_bf16x2((o[c * 32 + i0 + 6] + __uint_as_float(v[i0 + 6])) * inv, (o[c * 32 + i0 + 7] + __uint_as_float(v[i0 + 7])) * inv);
+              u.x = pack_bf16x2(__uint_as_float(v[i0 + 0]) * inv, __uint_as_float(v[i0 + 1]) * inv);
+              u.y = pack_bf16x2(__uint_as_float(v[i0 + 2]) * inv, __uint_as_float(v[i0 + 3]) * inv);
+              u.z = pack_bf16x2(__uint_as_float(v[i0 + 4]) * inv, __uint_as_float(v[i0 + 5]) * inv);
+              u.w = pack_bf16x2(__uint_as_float(v[i0 + 6]) * inv, __uint_as_float(v[i0 + 7]) * inv);
               reinterpret_cast<uint4*>(orow + c * 32)[q4] = u;
             }
           }
         }
-        if (hf == 0 && qi < g.Sq) lse[((long long)b * g.Hq + hq) * g.Sq + qi] = (l > 0.f) ? m * g.scale + logf(l) : -INFINITY;
+        if (row_ok) *lrow = l > 0.f ? m * g.scale + logf(l) : -INFINITY;
       }
-    } else if (qi < g.Sq) {
-      __nv_bfloat16* orow = out + (long long)qi * g.o_s + (long long)b * g.o_b + (long long)hq * g.o_h + hf * 64;
-      for (int i = 0; i < 64 / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0, 0, 0, 0);
-      if (hf == 0) lse[((long long)b * g.Hq + hq) * g.Sq + qi] = -INFINITY;
+    } else if (row_ok) {
+      for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0, 0, 0, 0);
+      *lrow = -INFINITY;
     }
   }
   tc_fence_before();
@@ -328,68 +449,122 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 }
 
 // ======================================================================= backward
-// delta[b, h, s] = sum_d dO * O
+// delta[b, h, s] = sum_d dO * O.  Half a warp per row (16 bytes per lane and operand), four rows
+// per half warp in flight; one block covers 64 consecutive rows of one head, so the results are
+// written as whole lines.
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                                                         float* __restrict__ delta, int B, int Hq, int Sq, long long do_s, long long do_b,
-                                                         long long do_h, long long o_s, long long o_b, long long o_h) {
-  const int wid = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int total = B * Hq * Sq;
-  if (wid >= total) return;
-  const int s = wid % Sq, h = (wid / Sq) % Hq, b = wid / (Sq * Hq);
-  const uint2* a = reinterpret_cast<const uint2*>(dout + s * do_s + b * do_b + h * do_h) + lane;
-  const uint2* c = reinterpret_cast<const uint2*>(out + s * o_s + b * o_b + h * o_h) + lane;
-  const uint2 av = *a, cv = *c;
-  float2 a0 = unpack_bf16x2(av.x), a1 = unpack_bf16x2(av.y), c0 = unpack_bf16x2(cv.x), c1 = unpack_bf16x2(cv.y);
-  float v = a0.x * c0.x + a0.y * c0.y + a1.x * c1.x + a1.y * c1.y;
+                                                         float* __restrict__ delta, int Hq, int S, long long do_s, long long do_b,
+                                                         long long do_h, long long o_s, long long o_b, long long o_h, int wide) {
+  const int hw = threadIdx.x >> 4, l16 = threadIdx.x & 15;
+  const int h = blockIdx.x % Hq, b = blockIdx.y;
+  const int s0 = (blockIdx.x / Hq) * 64 + hw * 4;
+  uint4 x[4], y[4];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) delta[((long long)b * Hq + h) * Sq + s] = v;
+  for (int i = 0; i < 4; ++i) {
+    const int s = min(s0 + i, S - 1);
+    x[i] = ld_nc_v4(dout + s * do_s + b * do_b + h * do_h + l16 * 8);
+    const __nv_bfloat16* o = out + s * o_s + b * o_b + h * o_h + l16 * 8;
+    if (wide) {
+      y[i] = ld_nc_v4(o);
+    } else {                              // O with rows that are only 8-byte aligned
+      const uint2 u = reinterpret_cast<const uint2*>(o)[0], v = reinterpret_cast<const uint2*>(o)[1];
+      y[i] = make_uint4(u.x, u.y, v.x, v.y);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float v = 0.f;
+    const uint32_t xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 p = unpack_bf16x2(xs[c]), q = unpack_bf16x2(ys[c]);
+      v += p.x * q.x + p.y * q.y;
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (l16 == 0 && s0 + i < S) delta[((long long)b * Hq + h) * S + s0 + i] = v;
+  }
 }
 
-struct BwdCtl {
-  uint64_t kv_full, qdo_full, qdo_empty, sdp_full, pds_ready, acc_full;
+// ----------------------------------------------------------------------- dK / dV
+constexpr int STAT_RING = 4;
+struct DkvCtl {
+  uint64_t k_full, v_full;
+  uint64_t q_full[2], q_empty[2], do_full[2], do_empty[2];
+  uint64_t stat_full[STAT_RING], stat_empty[STAT_RING];
+  uint64_t s_full, p_ready[2], dp_full, ds_ready[2], acc_full;      // [half of the query columns]
   uint32_t tmem_base;
   int abort_flag;
 };
-constexpr int BWD_SMEM = TILE_BYTES * 6 + 1024 + 256;     // K, V, Q, dO, P, dS
+constexpr int STAT_BYTES = STAT_RING * 2 * BQ * 4;                    // -lse * log2(e) and -delta of the query block
+constexpr int DKV_SMEM = TILE_BYTES * 6 + STAT_BYTES + 1024 + 512;    // K, V, Q x2, dO x2
 
-struct BwdGeometry {
-  int B, Hq, Hk, Sq, Sk, causal;
-  float scale;
+struct DkvArgs {
+  const float* lse;
+  const float* delta;
+  __nv_bfloat16* dk;
+  __nv_bfloat16* dv;
   long long dk_s, dk_b, dk_h, dv_s, dv_b, dv_h;
-  // Head split: the query heads of one KV head are divided over `hs` CTAs (grid.y = Hk * hs) when
+  // Head split: the query heads of one KV head are divided over `hs` CTAs (work heads = Hk * hs) when
   // KV blocks x batch x KV heads alone would leave SMs idle (tensor parallelism leaves one KV head per
-  // GPU).  Each CTA then writes fp32 partial dV / dK to `part` ([2][hs][Sk][B][Hk][128]) and
+  // GPU).  Each CTA then writes fp32 partial dV / dK to `part` ([2][hs][Tk][B][Hk][128]) and
   // attn_dkv_reduce_kernel adds them up.
   int hs;
   float* part;
-  DeviceStatus* status;
-  int x0, p0, ny;                 // as in Geometry; ny = Hk * hs
 };
 
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                const __grid_constant__ CUtensorMap tdo, const float* __restrict__ lse, const float* __restrict__ delta,
-                __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, const BwdGeometry g) {
+// Columns 32 c .. 32 c + 31 of this thread's accumulator rows of dV and dK -> memory.
+__device__ __forceinline__ void store_dkv_cols(const DkvArgs& a, float scale, const uint32_t (&x)[32], const uint32_t (&y)[32], float* pdv, float* pdk,
+                                               __nv_bfloat16* dvr, __nv_bfloat16* dkr) {
+  if (a.hs > 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      reinterpret_cast<float4*>(pdv)[j] = make_float4(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 2]),
+                                                      __uint_as_float(x[4 * j + 3]));
+      reinterpret_cast<float4*>(pdk)[j] = make_float4(__uint_as_float(y[4 * j]) * scale, __uint_as_float(y[4 * j + 1]) * scale,
+                                                      __uint_as_float(y[4 * j + 2]) * scale, __uint_as_float(y[4 * j + 3]) * scale);
+    }
+    return;
+  }
+#pragma unroll
+  for (int q4 = 0; q4 < 4; ++q4) {
+    uint4 u, w;
+    const int i0 = q4 * 8;
+    u.x = pack_bf16x2(__uint_as_float(x[i0]), __uint_as_float(x[i0 + 1]));
+    u.y = pack_bf16x2(__uint_as_float(x[i0 + 2]), __uint_as_float(x[i0 + 3]));
+    u.z = pack_bf16x2(__uint_as_float(x[i0 + 4]), __uint_as_float(x[i0 + 5]));
+    u.w = pack_bf16x2(__uint_as_float(x[i0 + 6]), __uint_as_float(x[i0 + 7]));
+    w.x = pack_bf16x2(__uint_as_float(y[i0]) * scale, __uint_as_float(y[i0 + 1]) * scale);
+    w.y = pack_bf16x2(__uint_as_float(y[i0 + 2]) * scale, __uint_as_float(y[i0 + 3]) * scale);
+    w.z = pack_bf16x2(__uint_as_float(y[i0 + 4]) * scale, __uint_as_float(y[i0 + 5]) * scale);
+    w.w = pack_bf16x2(__uint_as_float(y[i0 + 6]) * scale, __uint_as_float(y[i0 + 7]) * scale);
+    reinterpret_cast<uint4*>(dvr)[q4] = u;
+    reinterpret_cast<uint4*>(dkr)[q4] = w;
+  }
+}
+
+template <class Table>
+__global__ void __launch_bounds__(THREADS, 1)
+attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                    const __grid_constant__ CUtensorMap tdo, const __grid_constant__ Geometry g, const __grid_constant__ DkvArgs a,
+                    const __grid_constant__ Table table) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = smem + TILE_BYTES;
   uint8_t* sQ = smem + 2 * TILE_BYTES;
-  uint8_t* sDO = smem + 3 * TILE_BYTES;
-  uint8_t* sP = smem + 4 * TILE_BYTES;
-  uint8_t* sDS = smem + 5 * TILE_BYTES;
-  BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem + 6 * TILE_BYTES);
+  uint8_t* sDO = smem + 4 * TILE_BYTES;
+  float* sStat = reinterpret_cast<float*>(smem + 6 * TILE_BYTES);   // [STAT_RING][2][BQ]
+  DkvCtl* ctl = reinterpret_cast<DkvCtl*>(smem + 6 * TILE_BYTES + STAT_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pyz = g.p0 + (int)blockIdx.y + (int)blockIdx.z * (int)gridDim.y;
-  const int by = pyz % g.ny;
-  const int kb = g.x0 + (int)blockIdx.x, hk = by / g.hs, hpart = by % g.hs, b = pyz / g.ny;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const Work w = find_work(g, table, g.x0 + (int)blockIdx.x);
+  const int kb = w.tile, hk = w.head / a.hs, hpart = w.head % a.hs;
   const int group = g.Hq / g.Hk;
-  const int gpp = group / g.hs;                 // query heads handled by this CTA
+  const int gpp = group / a.hs;                 // query heads handled by this CTA
   const int hq0 = hk * group + hpart * gpp;
-  const int off = g.Sk - g.Sq;
-  const int nqb = (g.Sq + BQ - 1) / BQ;
+  const int off = w.nk - w.nq;
+  const int nqb = (w.nq + BQ - 1) / BQ;
   // first query block that sees any key of this block: i + off >= kb*BKV
   int qb0 = 0;
   if (g.causal) {
@@ -399,264 +574,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const int n_iter = qb0 < nqb ? (nqb - qb0) * gpp : 0;
 
   if (threadIdx.x == 0) {
-    mbar_init(&ctl->kv_full, 1); mbar_init(&ctl->qdo_full, 1); mbar_init(&ctl->qdo_empty, 1);
-    mbar_init(&ctl->sdp_full, 1); mbar_init(&ctl->pds_ready, 8); mbar_init(&ctl->acc_full, 1);
-    ctl->abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) { tmem_alloc(&ctl->tmem_base, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = ctl->tmem_base;
-  volatile int* abort_flag = &ctl->abort_flag;
-  // TMEM columns: [0,128) S, [128,256) dP, [256,384) dV, [384,512) dK
-
-  if (warp == 0) {
-    if (lane == 0 && n_iter > 0) {
-      tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv); tma_prefetch_desc(&tdo);
-      mbar_expect_tx(&ctl->kv_full, 2 * TILE_BYTES);
-      tma_load_4d(sK, &tk, &ctl->kv_full, 0, hk, b, kb * BKV);
-      tma_load_4d(sK + HALF_BYTES, &tk, &ctl->kv_full, 64, hk, b, kb * BKV);
-      tma_load_4d(sV, &tv, &ctl->kv_full, 0, hk, b, kb * BKV);
-      tma_load_4d(sV + HALF_BYTES, &tv, &ctl->kv_full, 64, hk, b, kb * BKV);
-      for (int it = 0; it < n_iter; ++it) {
-        const int hq = hq0 + it % gpp;
-        const int qb = qb0 + it / gpp;
-        if (!mbar_wait(&ctl->qdo_empty, (it & 1) ^ 1, abort_flag, g.status, 500)) break;
-        mbar_expect_tx(&ctl->qdo_full, 2 * TILE_BYTES);
-        tma_load_4d(sQ, &tq, &ctl->qdo_full, 0, hq, b, qb * BQ);
-        tma_load_4d(sQ + HALF_BYTES, &tq, &ctl->qdo_full, 64, hq, b, qb * BQ);
-        tma_load_4d(sDO, &tdo, &ctl->qdo_full, 0, hq, b, qb * BQ);
-        tma_load_4d(sDO + HALF_BYTES, &tdo, &ctl->qdo_full, 64, hq, b, qb * BQ);
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0 && n_iter > 0) {
-      constexpr uint32_t id_kk = umma_idesc_bf16(128, 128, 0, 0);   // S, dP: both operands K-major
-      constexpr uint32_t id_mm = umma_idesc_bf16(128, 128, 1, 1);   // dV, dK: both operands MN-major
-      const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), q_base = smem_u32(sQ), do_base = smem_u32(sDO);
-      const uint32_t p_base = smem_u32(sP), ds_base = smem_u32(sDS);
-      bool ok = mbar_wait(&ctl->kv_full, 0, abort_flag, g.status, 510);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const uint32_t ph = it & 1;
-        if (!mbar_wait(&ctl->qdo_full, ph, abort_flag, g.status, 511)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 0, desc_kmajor(q_base, kk), desc_kmajor(k_base, kk), id_kk, kk > 0);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 128, desc_kmajor(do_base, kk), desc_kmajor(v_base, kk), id_kk, kk > 0);
-        umma_commit(&ctl->sdp_full);
-        if (!mbar_wait(&ctl->pds_ready, ph, abort_flag, g.status, 513)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 256, desc_mnmajor(p_base, kk), desc_mnmajor(do_base, kk), id_mm, (it | kk) != 0);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 384, desc_mnmajor(ds_base, kk), desc_mnmajor(q_base, kk), id_mm, (it | kk) != 0);
-        umma_commit(&ctl->qdo_empty);           // Q and dO are free once dV and dK have read them
-      }
-      if (ok) umma_commit(&ctl->acc_full);
-    }
-    __syncwarp();
-  } else {
-    // warps 2..5 and 6..9 cover the four TMEM lane quarters twice: the first set works on
-    // columns [0, 64), the second on [64, 128) of every 128-column tile
-    const int quarter = warp & 3;
-    const int c_lo = ((warp - 2) >> 2) * 2;
-    const int r = quarter * 32 + lane;
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const float sl2 = g.scale * LOG2E;
-    bool ok = n_iter > 0;
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const uint32_t ph = it & 1;
-      const int hq = hq0 + it % gpp;
-      const int qb = qb0 + it / gpp;
-      const int qi = qb * BQ + r;
-      const bool row_ok = qi < g.Sq;
-      const long long stat = ((long long)b * g.Hq + hq) * g.Sq + qi;
-      const float L = row_ok ? lse[stat] * LOG2E : 0.f;
-      const float dl = row_ok ? delta[stat] : 0.f;
-      if (!mbar_wait(&ctl->sdp_full, ph, abort_flag, g.status, 520)) { ok = false; break; }
-      tc_fence_after();
-      const int key0 = kb * BKV;
-      int limit = g.Sk - key0;
-      if (g.causal) limit = min(limit, qi + off - key0 + 1);
-      if (!row_ok) limit = 0;
-#pragma unroll 1
-      for (int c = c_lo; c < c_lo + 2; ++c) {
-        uint32_t sv[32], dpv[32];
-        tmem_ld32(tmem + 0 + lane_base + c * 32, sv);
-        tmem_ld32(tmem + 128 + lane_base + c * 32, dpv);
-        tmem_ld_wait();
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          float p[8], ds[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int col = c * 32 + q4 * 8 + i;
-            float pe = exp2f(__uint_as_float(sv[q4 * 8 + i]) * sl2 - L);
-            if (col >= limit) pe = 0.f;
-            p[i] = pe;
-            ds[i] = pe * (__uint_as_float(dpv[q4 * 8 + i]) - dl);
-          }
-          uint4 up, ud;
-          up.x = pack_bf16x2(p[0], p[1]); up.y = pack_bf16x2(p[2], p[3]); up.z = pack_bf16x2(p[4], p[5]); up.w = pack_bf16x2(p[6], p[7]);
-          ud.x = pack_bf16x2(ds[0], ds[1]); ud.y = pack_bf16x2(ds[2], ds[3]); ud.z = pack_bf16x2(ds[4], ds[5]); ud.w = pack_bf16x2(ds[6], ds[7]);
-          const uint32_t o = swz_off(r, c * 4 + q4);
-          *reinterpret_cast<uint4*>(sP + o) = up;
-          *reinterpret_cast<uint4*>(sDS + o) = ud;
-        }
-      }
-      tc_fence_before();
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->pds_ready);
-    }
-    // dK (times scale) and dV of this key block
-    const int kj = kb * BKV + r;
-    // fp32 partial rows of this CTA's head part (head split only)
-    const long long part_elems = (long long)g.Sk * g.B * g.Hk * D;
-    float* pdv = g.hs > 1 ? g.part + (long long)hpart * part_elems + (((long long)kj * g.B + b) * g.Hk + hk) * D : nullptr;
-    float* pdk = g.hs > 1 ? pdv + (long long)g.hs * part_elems : nullptr;
-    if (g.hs > 1) {
-      if (ok && n_iter > 0) {
-        if (mbar_wait(&ctl->acc_full, 0, abort_flag, g.status, 523)) {
-          tc_fence_after();
-#pragma unroll 1
-          for (int c = c_lo; c < c_lo + 2; ++c) {
-            uint32_t a[32], bb[32];
-            tmem_ld32(tmem + 256 + lane_base + c * 32, a);      // warp-collective: no per-lane branch around it
-            tmem_ld32(tmem + 384 + lane_base + c * 32, bb);
-            tmem_ld_wait();
-            if (kj < g.Sk) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                reinterpret_cast<float4*>(pdv + c * 32)[j] = make_float4(__uint_as_float(a[4 * j]), __uint_as_float(a[4 * j + 1]),
-                                                                         __uint_as_float(a[4 * j + 2]), __uint_as_float(a[4 * j + 3]));
-                reinterpret_cast<float4*>(pdk + c * 32)[j] =
-                    make_float4(__uint_as_float(bb[4 * j]) * g.scale, __uint_as_float(bb[4 * j + 1]) * g.scale,
-                                __uint_as_float(bb[4 * j + 2]) * g.scale, __uint_as_float(bb[4 * j + 3]) * g.scale);
-              }
-            }
-          }
-        }
-      } else if (n_iter == 0 && kj < g.Sk) {
-        for (int i = c_lo * 8; i < c_lo * 8 + 16; ++i) {
-          reinterpret_cast<float4*>(pdv)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          reinterpret_cast<float4*>(pdk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-    } else if (ok && n_iter > 0) {
-      if (mbar_wait(&ctl->acc_full, 0, abort_flag, g.status, 522)) {
-        tc_fence_after();
-        __nv_bfloat16* dvr = dv + (long long)kj * g.dv_s + (long long)b * g.dv_b + (long long)hk * g.dv_h;
-        __nv_bfloat16* dkr = dk + (long long)kj * g.dk_s + (long long)b * g.dk_b + (long long)hk * g.dk_h;
-#pragma unroll 1
-        for (int c = c_lo; c < c_lo + 2; ++c) {
-          uint32_t a[32], bb[32];
-          tmem_ld32(tmem + 256 + lane_base + c * 32, a);
-          tmem_ld32(tmem + 384 + lane_base + c * 32, bb);
-          tmem_ld_wait();
-          if (kj < g.Sk) {
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-              uint4 u, w;
-              const int i0 = q4 * 8;
-              u.x = pack_bf16x2(__uint_as_float(a[i0]), __uint_as_float(a[i0 + 1]));
-              u.y = pack_bf16x2(__uint_as_float(a[i0 + 2]), __uint_as_float(a[i0 + 3]));
-              u.z = pack_bf16x2(__uint_as_float(a[i0 + 4]), __uint_as_float(a[i0 + 5]));
-              u.w = pack_bf16x2(__uint_as_float(a[i0 + 6]), __uint_as_float(a[i0 + 7]));
-              w.x = pack_bf16x2(__uint_as_float(bb[i0]) * g.scale, __uint_as_float(bb[i0 + 1]) * g.scale);
-              w.y = pack_bf16x2(__uint_as_float(bb[i0 + 2]) * g.scale, __uint_as_float(bb[i0 + 3]) * g.scale);
-              w.z = pack_bf16x2(__uint_as_float(bb[i0 + 4]) * g.scale, __uint_as_float(bb[i0 + 5]) * g.scale);
-              w.w = pack_bf16x2(__uint_as_float(bb[i0 + 6]) * g.scale, __uint_as_float(bb[i0 + 7]) * g.scale);
-              reinterpret_cast<uint4*>(dvr + c * 32)[q4] = u;
-              reinterpret_cast<uint4*>(dkr + c * 32)[q4] = w;
-            }
-          }
-        }
-      }
-    } else if (n_iter == 0 && kj < g.Sk && c_lo == 0) {
-      __nv_bfloat16* dvr = dv + (long long)kj * g.dv_s + (long long)b * g.dv_b + (long long)hk * g.dv_h;
-      __nv_bfloat16* dkr = dk + (long long)kj * g.dk_s + (long long)b * g.dk_b + (long long)hk * g.dk_h;
-      for (int i = 0; i < D / 8; ++i) {
-        reinterpret_cast<uint4*>(dvr)[i] = make_uint4(0, 0, 0, 0);
-        reinterpret_cast<uint4*>(dkr)[i] = make_uint4(0, 0, 0, 0);
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
-}
-
-// ----------------------------------------------------------------------- backward, dK/dV, pipelined form
-// Same work split as attn_bwd_kernel (one CTA per 128 keys, loop over the query heads of its
-// part of the KV group and over the query blocks that see these keys), rearranged so that the
-// tensor cores, the TMA and the math warps overlap:
-//   * the scores are formed transposed, S^T = K Q^T and dP^T = V dO^T (keys on the TMEM lanes,
-//     64 queries per iteration on the columns), double-buffered in TMEM (4 x 64 columns), so the
-//     products of iteration i+1 run while the math warps work on iteration i;
-//   * a math thread owns one key row: it forms P^T = exp2(S^T - lse[q]) and dS^T = P^T (dP^T -
-//     delta[q]) with the per-query statistics taken from registers of its warp (shuffles), and
-//     writes its 64-byte piece of the row into a K-major [128 keys][64 queries] shared-memory
-//     tile, which is the A operand of dV += P^T dO and dK += dS^T Q as it stands;
-//   * Q / dO tiles are 64 rows (16 KiB each) in a 2-stage ring, P^T / dS^T tiles likewise, which
-//     fits 192 KiB; the TMA for iteration i+1 is in flight during iteration i.
-// dV / dK accumulate in TMEM columns [256, 512) exactly as in attn_bwd_kernel, so the epilogue
-// (bf16 rows, or fp32 partials under the head split) is the same.
-constexpr int BQT = 64;                          // queries per iteration
-constexpr int QT_HALF = BQT * 128;               // one [64 rows][64 elems] swizzled box
-constexpr int QT_TILE = 2 * QT_HALF;             // [64][128] bf16
-constexpr int PT_TILE = BKV * 128;               // [128 keys][64 queries] bf16, one 128-byte row per key
-struct BwdTCtl {
-  uint64_t kv_full, qdo_full[2], stage_free[2], sdp_full[2], sdp_empty[2], pds_ready[2], acc_full;
-  uint32_t tmem_base;
-  int abort_flag;
-};
-constexpr int BWDT_SMEM = 2 * TILE_BYTES + 4 * QT_TILE + 4 * PT_TILE + 1024 + 256;
-
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_t_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                  const __grid_constant__ CUtensorMap tdo, const float* __restrict__ lse, const float* __restrict__ delta,
-                  __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, const BwdGeometry g) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem;
-  uint8_t* sV = smem + TILE_BYTES;
-  uint8_t* sQ = smem + 2 * TILE_BYTES;                     // 2 stages
-  uint8_t* sDO = sQ + 2 * QT_TILE;                         // 2 stages
-  uint8_t* sP = sDO + 2 * QT_TILE;                         // 2 stages
-  uint8_t* sDS = sP + 2 * PT_TILE;                         // 2 stages
-  BwdTCtl* ctl = reinterpret_cast<BwdTCtl*>(sDS + 2 * PT_TILE);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pyz = g.p0 + (int)blockIdx.y + (int)blockIdx.z * (int)gridDim.y;
-  const int by = pyz % g.ny;
-  const int kb = g.x0 + (int)blockIdx.x, hk = by / g.hs, hpart = by % g.hs, b = pyz / g.ny;
-  const int group = g.Hq / g.Hk;
-  const int gpp = group / g.hs;
-  const int hq0 = hk * group + hpart * gpp;
-  const int off = g.Sk - g.Sq;
-  const int nqb = (g.Sq + BQT - 1) / BQT;
-  int qb0 = 0;
-  if (g.causal) {
-    const int first_q = kb * BKV - off;
-    qb0 = first_q <= 0 ? 0 : first_q / BQT;
-  }
-  const int n_iter = qb0 < nqb ? (nqb - qb0) * gpp : 0;
-
-  if (threadIdx.x == 0) {
-    mbar_init(&ctl->kv_full, 1);
-    mbar_init(&ctl->acc_full, 1);
+    mbar_init(&ctl->k_full, 1); mbar_init(&ctl->v_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&ctl->qdo_full[i], 1);
-      mbar_init(&ctl->stage_free[i], 1);
-      mbar_init(&ctl->sdp_full[i], 1);
-      mbar_init(&ctl->sdp_empty[i], 8);
-      mbar_init(&ctl->pds_ready[i], 8);
+      mbar_init(&ctl->q_full[i], 1); mbar_init(&ctl->q_empty[i], 1);
+      mbar_init(&ctl->do_full[i], 1); mbar_init(&ctl->do_empty[i], 1);
     }
+    for (int i = 0; i < STAT_RING; ++i) { mbar_init(&ctl->stat_full[i], 1); mbar_init(&ctl->stat_empty[i], 8); }
+    mbar_init(&ctl->s_full, 1); mbar_init(&ctl->dp_full, 1); mbar_init(&ctl->acc_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&ctl->p_ready[i], 8); mbar_init(&ctl->ds_ready[i], 8); }
     ctl->abort_flag = 0;
     mbar_fence_init();
   }
@@ -664,202 +589,228 @@ attn_bwd_t_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort_flag;
-  // TMEM columns: S^T buffers [0,64) [64,128); dP^T buffers [128,192) [192,256); dV [256,384); dK [384,512)
+  // TMEM columns: [0,128) S^T, [128,256) dP^T, [256,384) dV, [384,512) dK.  A math warp covers 64 of the 128 query
+  // columns and packs its bf16 P^T (dS^T) into the first 32 of the 64 columns it has read.
 
   if (warp == 0) {
     if (lane == 0 && n_iter > 0) {
       tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv); tma_prefetch_desc(&tdo);
-      mbar_expect_tx(&ctl->kv_full, 2 * TILE_BYTES);
-      tma_load_4d(sK, &tk, &ctl->kv_full, 0, hk, b, kb * BKV);
-      tma_load_4d(sK + HALF_BYTES, &tk, &ctl->kv_full, 64, hk, b, kb * BKV);
-      tma_load_4d(sV, &tv, &ctl->kv_full, 0, hk, b, kb * BKV);
-      tma_load_4d(sV + HALF_BYTES, &tv, &ctl->kv_full, 64, hk, b, kb * BKV);
+      mbar_expect_tx(&ctl->k_full, TILE_BYTES);
+      load_tile(sK, &tk, &ctl->k_full, hk, w.b, w.k0 + kb * BKV);
+      int hq = hq0, row = w.q0 + qb0 * BQ;
       for (int it = 0; it < n_iter; ++it) {
         const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        const int hq = hq0 + it % gpp;
-        const int qb = qb0 + it / gpp;
-        if (!mbar_wait(&ctl->stage_free[st], ph ^ 1, abort_flag, g.status, 530)) break;
-        mbar_expect_tx(&ctl->qdo_full[st], 2 * QT_TILE);
-        uint8_t* q_dst = sQ + st * QT_TILE;
-        uint8_t* do_dst = sDO + st * QT_TILE;
-        tma_load_4d(q_dst, &tq, &ctl->qdo_full[st], 0, hq, b, qb * BQT);
-        tma_load_4d(q_dst + QT_HALF, &tq, &ctl->qdo_full[st], 64, hq, b, qb * BQT);
-        tma_load_4d(do_dst, &tdo, &ctl->qdo_full[st], 0, hq, b, qb * BQT);
-        tma_load_4d(do_dst + QT_HALF, &tdo, &ctl->qdo_full[st], 64, hq, b, qb * BQT);
+        const uint32_t ph = ((it >> 1) & 1) ^ 1;
+        if (!mbar_wait(&ctl->q_empty[st], ph, abort_flag, g.status, 500)) break;
+        mbar_expect_tx(&ctl->q_full[st], TILE_BYTES);
+        load_tile(sQ + st * TILE_BYTES, &tq, &ctl->q_full[st], hq, w.b, row);
+        if (it == 0) {
+          mbar_expect_tx(&ctl->v_full, TILE_BYTES);
+          load_tile(sV, &tv, &ctl->v_full, hk, w.b, w.k0 + kb * BKV);
+        }
+        if (!mbar_wait(&ctl->do_empty[st], ph, abort_flag, g.status, 501)) break;
+        mbar_expect_tx(&ctl->do_full[st], TILE_BYTES);
+        load_tile(sDO + st * TILE_BYTES, &tdo, &ctl->do_full[st], hq, w.b, row);
+        if (++hq == hq0 + gpp) { hq = hq0; row += BQ; }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && n_iter > 0) {
-      constexpr uint32_t id_st = umma_idesc_bf16(128, BQT, 0, 0);    // S^T, dP^T: A = K / V (K-major), B = Q / dO (K-major), N = 64
-      constexpr uint32_t id_acc = umma_idesc_bf16(128, 128, 0, 1);   // dV, dK: A = P^T / dS^T (K-major), B = dO / Q (MN-major)
+    const uint32_t leader = elect_one();
+    if (n_iter > 0) {
+      constexpr uint32_t id_st = umma_idesc_bf16(128, 128, 0, 0);    // S^T, dP^T: A = K / V, B = Q / dO, both K-major
+      constexpr uint32_t id_acc = umma_idesc_bf16(128, 128, 0, 1);   // dV, dK: A = P^T / dS^T in TMEM, B = dO / Q MN-major
       const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV);
-      bool ok = mbar_wait(&ctl->kv_full, 0, abort_flag, g.status, 540);
-      // S^T and dP^T of iteration j into TMEM buffer j & 1
-      auto issue_scores = [&](int j) -> bool {
+      // scores of iteration j: A = K (V), B = the query block of Q (dO)
+      auto issue_scores = [&](int j, bool dp) -> bool {
         const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&ctl->qdo_full[st], ph, abort_flag, g.status, 541)) return false;
-        if (!mbar_wait(&ctl->sdp_empty[st], ph ^ 1, abort_flag, g.status, 542)) return false;
+        if (!warp_wait(dp ? &ctl->do_full[st] : &ctl->q_full[st], (j >> 1) & 1, abort_flag, g.status, dp ? 512 : 511)) return false;
+        uint8_t* tile = (dp ? sDO : sQ) + st * TILE_BYTES;
+        if (sizeof(Table) > 1 && w.q0 + w.nq < g.Tq) {
+          const int rows = w.nq - (qb0 + j / gpp) * BQ;
+          if (rows < BQ) zero_tile_rows(tile, rows, lane);
+        }
         tc_fence_after();
-        const uint32_t q_base = smem_u32(sQ + st * QT_TILE), do_base = smem_u32(sDO + st * QT_TILE);
+        {
+          const uint32_t b_base = smem_u32(tile), a_base = dp ? v_base : k_base, d = tmem + (dp ? 128 : 0);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem + 64 * st, desc_kmajor(k_base, kk), umma_smem_desc(q_base + (kk >> 2) * QT_HALF + (kk & 3) * 32, 16, 1024), id_st,
-                    kk > 0);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem + 128 + 64 * st, desc_kmajor(v_base, kk), umma_smem_desc(do_base + (kk >> 2) * QT_HALF + (kk & 3) * 32, 16, 1024),
-                    id_st, kk > 0);
-        umma_commit(&ctl->sdp_full[st]);
+          for (int kk = 0; kk < 8; ++kk) umma_bf16_by(leader, d, desc_kmajor(a_base, kk), desc_kmajor(b_base, kk), id_st, kk > 0);
+          umma_commit_by(leader, dp ? &ctl->dp_full : &ctl->s_full);
+        }
         return true;
       };
-      if (ok) ok = issue_scores(0);
+      // gradient of iteration j: dV += P^T dO (dK += dS^T Q).  Each math warp delivers its 64 query columns in two parts
+      // of 32, so the products of the first parts run beside the math of the second.
+      auto issue_grad = [&](int j, bool dk) -> bool {
+        const uint32_t b_base = smem_u32((dk ? sQ : sDO) + (j & 1) * TILE_BYTES), src = tmem + (dk ? 128 : 0), d = tmem + (dk ? 384 : 256);
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          if (!warp_wait(dk ? &ctl->ds_ready[part] : &ctl->p_ready[part], j & 1, abort_flag, g.status, dk ? 514 : 513)) return false;
+          tc_fence_after();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int half = i >> 1, kk = 4 * half + 2 * part + (i & 1);        // step kk of the contraction = 8 TMEM columns
+            umma_bf16_ts_by(leader, d, src + half * 64 + (kk & 3) * 8, desc_mnmajor(b_base, kk), id_acc, (j | part | i) != 0);
+          }
+        }
+        umma_commit_by(leader, dk ? &ctl->q_empty[j & 1] : &ctl->do_empty[j & 1]);
+        return true;
+      };
+      bool ok = warp_wait(&ctl->k_full, 0, abort_flag, g.status, 510) && issue_scores(0, false) &&
+                warp_wait(&ctl->v_full, 0, abort_flag, g.status, 510) && issue_scores(0, true);
       for (int it = 0; it < n_iter && ok; ++it) {
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        if (it + 1 < n_iter && !issue_scores(it + 1)) { ok = false; break; }
-        if (!mbar_wait(&ctl->pds_ready[st], ph, abort_flag, g.status, 543)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t p_base = smem_u32(sP + st * PT_TILE), ds_base = smem_u32(sDS + st * PT_TILE);
-        const uint32_t q_base = smem_u32(sQ + st * QT_TILE), do_base = smem_u32(sDO + st * QT_TILE);
-#pragma unroll
-        for (int kk = 0; kk < BQT / 16; ++kk)
-          umma_bf16(tmem + 256, umma_smem_desc(p_base + kk * 32, 16, 1024), umma_smem_desc(do_base + kk * 2048, QT_HALF, 1024), id_acc,
-                    (it | kk) != 0);
-#pragma unroll
-        for (int kk = 0; kk < BQT / 16; ++kk)
-          umma_bf16(tmem + 384, umma_smem_desc(ds_base + kk * 32, 16, 1024), umma_smem_desc(q_base + kk * 2048, QT_HALF, 1024), id_acc,
-                    (it | kk) != 0);
-        umma_commit(&ctl->stage_free[st]);      // Q, dO, P^T, dS^T of this stage are free once dV and dK have read them
+        // a score product goes in order behind the gradient product that reads the same TMEM columns
+        ok = issue_grad(it, false) && (it + 1 >= n_iter || issue_scores(it + 1, false)) && issue_grad(it, true) &&
+             (it + 1 >= n_iter || issue_scores(it + 1, true));
       }
-      if (ok) umma_commit(&ctl->acc_full);
+      if (ok) umma_commit_by(leader, &ctl->acc_full);
     }
     __syncwarp();
-  } else {
-    // warps 2..5 take query columns [0, 32) of the 64-column buffers, warps 6..9 take [32, 64);
-    // each warp covers the TMEM lane quarter (key rows) it is allowed to read
-    const int quarter = warp & 3;
-    const int c_half = (warp - 2) >> 2;
-    const int r = quarter * 32 + lane;                 // key row inside the block
-    const int kv_g = kb * BKV + r;
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const float sl2 = g.scale * LOG2E;
-    bool ok = n_iter > 0;
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int st = it & 1;
-      const uint32_t ph = (it >> 1) & 1;
-      const int hq = hq0 + it % gpp;
-      const int qb = qb0 + it / gpp;
-      // lane j holds the statistics of query column j of this warp's 32 columns
-      const int q_mine = qb * BQT + c_half * 32 + lane;
-      const bool q_ok = q_mine < g.Sq;
-      const long long stat = ((long long)b * g.Hq + hq) * g.Sq + q_mine;
-      const float L_mine = q_ok ? lse[stat] * LOG2E : INFINITY;     // +inf: exp2(x - inf) = 0 for rows past the end
-      const float d_mine = q_ok ? delta[stat] : 0.f;
-      if (!mbar_wait(&ctl->sdp_full[st], ph, abort_flag, g.status, 550)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t sv[32], dpv[32];
-      tmem_ld32(tmem + 64 * st + lane_base + c_half * 32, sv);
-      tmem_ld32(tmem + 128 + 64 * st + lane_base + c_half * 32, dpv);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->sdp_empty[st]);              // this TMEM buffer may take iteration it + 2
-      uint32_t pk[16], dsk[16];
-      const int q0 = qb * BQT + c_half * 32;
+  } else if (warp == 2) {
+    // statistics of the query blocks, ahead of the math warps.  Rows past the end get -inf: exp2(x - inf) = 0.
+    int hq = hq0, q0 = qb0 * BQ;
+    for (int it = 0; it < n_iter; ++it) {
+      const int st = it % STAT_RING;
+      const uint32_t ph = ((it / STAT_RING) & 1) ^ 1;
+      const float* lp = a.lse + ((long long)w.sid * g.Hq + hq) * g.ls;
+      const float* dp = a.delta + ((long long)w.b * g.Hq + hq) * g.Tq + w.q0;
+      float L[4], dl[4];
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        float pe[2], de[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float Lq = __shfl_sync(0xffffffffu, L_mine, j + e);
-          const float dq_ = __shfl_sync(0xffffffffu, d_mine, j + e);
-          const bool valid = kv_g < g.Sk && (!g.causal || kv_g <= q0 + j + e + off);
-          const float p = valid ? exp2f(__uint_as_float(sv[j + e]) * sl2 - Lq) : 0.f;
-          pe[e] = p;
-          de[e] = p * (__uint_as_float(dpv[j + e]) - dq_);
-        }
-        pk[j >> 1] = pack_bf16x2(pe[0], pe[1]);
-        dsk[j >> 1] = pack_bf16x2(de[0], de[1]);
+      for (int i = 0; i < 4; ++i) {
+        const int q = q0 + i * 32 + lane;
+        L[i] = q < w.nq ? -lp[q] * LOG2E : -INFINITY;
+        dl[i] = q < w.nq ? -dp[q] : 0.f;
       }
-      if (!mbar_wait(&ctl->stage_free[st], ph ^ 1, abort_flag, g.status, 551)) { ok = false; break; }
-      uint8_t* prow = sP + st * PT_TILE + r * 128;
-      uint8_t* drow = sDS + st * PT_TILE + r * 128;
+      if (!mbar_wait(&ctl->stat_empty[st], ph, abort_flag, g.status, 515)) break;
+      float* dst = sStat + st * 2 * BQ;
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint32_t o = (uint32_t)(((c_half * 4 + t) ^ (r & 7)) << 4);
-        *reinterpret_cast<uint4*>(prow + o) = make_uint4(pk[4 * t], pk[4 * t + 1], pk[4 * t + 2], pk[4 * t + 3]);
-        *reinterpret_cast<uint4*>(drow + o) = make_uint4(dsk[4 * t], dsk[4 * t + 1], dsk[4 * t + 2], dsk[4 * t + 3]);
+      for (int i = 0; i < 4; ++i) {
+        dst[i * 32 + lane] = L[i];
+        dst[BQ + i * 32 + lane] = dl[i];
       }
-      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->pds_ready[st]);
+      if (lane == 0) mbar_arrive(&ctl->stat_full[st]);
+      if (++hq == hq0 + gpp) { hq = hq0; q0 += BQ; }
     }
-    // epilogue: this thread's key row of dV and dK, columns [64 * c_half, 64 * c_half + 64)
-    const int c_lo = c_half * 2;
-    const int kj = kv_g;
-    const long long part_elems = (long long)g.Sk * g.B * g.Hk * D;
-    float* pdv = g.hs > 1 ? g.part + (long long)hpart * part_elems + (((long long)kj * g.B + b) * g.Hk + hk) * D : nullptr;
-    float* pdk = g.hs > 1 ? pdv + (long long)g.hs * part_elems : nullptr;
-    if (ok && n_iter > 0) {
-      if (mbar_wait(&ctl->acc_full, 0, abort_flag, g.status, 552)) {
-        tc_fence_after();
-        __nv_bfloat16* dvr = dv + (long long)kj * g.dv_s + (long long)b * g.dv_b + (long long)hk * g.dv_h;
-        __nv_bfloat16* dkr = dk + (long long)kj * g.dk_s + (long long)b * g.dk_b + (long long)hk * g.dk_h;
-#pragma unroll 1
-        for (int c = c_lo; c < c_lo + 2; ++c) {
-          uint32_t a[32], bb[32];
-          tmem_ld32(tmem + 256 + lane_base + c * 32, a);
-          tmem_ld32(tmem + 384 + lane_base + c * 32, bb);
-          tmem_ld_wait();
-          if (kj >= g.Sk) continue;
-          if (g.hs > 1) {
+  } else if (warp >= MATH_WARP0) {
+    const int quarter = warp & 3;
+    const int half = (warp - MATH_WARP0) >> 2;         // query columns [64 half, 64 half + 64)
+    const int kj = kb * BKV + quarter * 32 + lane;     // this thread's key
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t ts = tmem + lane_base + half * 64, tp = ts + 128;
+    const float sl2 = g.scale * LOG2E;
+    const uint64_t sl2_2 = pk2(sl2, sl2);
+    bool ok = n_iter > 0;
+    int qb = qb0, head = 0;                            // iterations walk the heads of a query block, then the next block
+    for (int it = 0; it < n_iter && ok; ++it) {
+      const int sst = it % STAT_RING;
+      const uint64_t* nL = reinterpret_cast<const uint64_t*>(sStat + sst * 2 * BQ + half * 64);
+      const uint64_t* nD = nL + BQ / 2;
+      // query column c of this warp is valid iff lo <= c < hi
+      const int qbase = qb * BQ + half * 64;
+      const bool edge = (qb + 1) * BQ > w.nq || (kb + 1) * BKV > w.nk || (g.causal && kb * BKV + BKV - 1 > qb * BQ + off);
+      const int lo = kj >= w.nk ? BQ : (g.causal ? kj - off - qbase : 0);
+      const int hi = w.nq - qbase;
+      if (!mbar_wait(&ctl->stat_full[sst], (it / STAT_RING) & 1, abort_flag, g.status, 520)) { ok = false; break; }
+      if (!mbar_wait(&ctl->s_full, it & 1, abort_flag, g.status, 521)) { ok = false; break; }
+      tc_fence_after();
+      // the mask is a path of its own: as predicates it costs more issue slots than the arithmetic
+      uint64_t p[32];
+      auto probabilities = [&](auto edge_) {
+        constexpr bool masked = decltype(edge_)::value;
+        uint32_t s[64];
+        tmem_ld32(ts, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+        tmem_ld32(ts + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
+        tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              reinterpret_cast<float4*>(pdv + c * 32)[j] = make_float4(__uint_as_float(a[4 * j]), __uint_as_float(a[4 * j + 1]),
-                                                                       __uint_as_float(a[4 * j + 2]), __uint_as_float(a[4 * j + 3]));
-              reinterpret_cast<float4*>(pdk + c * 32)[j] =
-                  make_float4(__uint_as_float(bb[4 * j]) * g.scale, __uint_as_float(bb[4 * j + 1]) * g.scale,
-                              __uint_as_float(bb[4 * j + 2]) * g.scale, __uint_as_float(bb[4 * j + 3]) * g.scale);
-            }
-          } else {
+        for (int c = 0; c < 2; ++c) {
+          uint32_t pk[16];
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-              uint4 u, w;
-              const int i0 = q4 * 8;
-              u.x = pack_bf16x2(__uint_as_float(a[i0]), __uint_as_float(a[i0 + 1]));
-              u.y = pack_bf16x2(__uint_as_float(a[i0 + 2]), __uint_as_float(a[i0 + 3]));
-              u.z = pack_bf16x2(__uint_as_float(a[i0 + 4]), __uint_as_float(a[i0 + 5]));
-              u.w = pack_bf16x2(__uint_as_float(a[i0 + 6]), __uint_as_float(a[i0 + 7]));
-              w.x = pack_bf16x2(__uint_as_float(bb[i0]) * g.scale, __uint_as_float(bb[i0 + 1]) * g.scale);
-              w.y = pack_bf16x2(__uint_as_float(bb[i0 + 2]) * g.scale, __uint_as_float(bb[i0 + 3]) * g.scale);
-              w.z = pack_bf16x2(__uint_as_float(bb[i0 + 4]) * g.scale, __uint_as_float(bb[i0 + 5]) * g.scale);
-              w.w = pack_bf16x2(__uint_as_float(bb[i0 + 6]) * g.scale, __uint_as_float(bb[i0 + 7]) * g.scale);
-              reinterpret_cast<uint4*>(dvr + c * 32)[q4] = u;
-              reinterpret_cast<uint4*>(dkr + c * 32)[q4] = w;
+          for (int i = 0; i < 16; i += 2) {
+            const ulonglong2 L = *reinterpret_cast<const ulonglong2*>(nL + c * 16 + i);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int e = c * 32 + 2 * (i + h);
+              float x, y;
+              upk2(fma2(pk2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sl2_2, h ? L.y : L.x), x, y);
+              x = ex2(x); y = ex2(y);
+              if (masked) {                            // also rows without statistics (lse = -inf) and neighbours' rows
+                if (e < lo || e >= hi) x = 0.f;
+                if (e + 1 < lo || e + 1 >= hi) y = 0.f;
+              }
+              p[c * 16 + i + h] = pk2(x, y);
+              pk[i + h] = pack_bf16x2(x, y);
             }
+          }
+          tmem_st16(ts + c * 16, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->p_ready[c]);
+        }
+      };
+      if (edge) probabilities(std::true_type{});
+      else probabilities(std::false_type{});
+      if (!mbar_wait(&ctl->dp_full, it & 1, abort_flag, g.status, 522)) { ok = false; break; }
+      tc_fence_after();
+      {
+        uint32_t v[64];
+        tmem_ld32(tp, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        tmem_ld32(tp + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            const ulonglong2 dl = *reinterpret_cast<const ulonglong2*>(nD + c * 16 + i);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int e = c * 32 + 2 * (i + h);
+              float x, y;
+              upk2(mul2(p[c * 16 + i + h], add2(pk2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), h ? dl.y : dl.x)), x, y);
+              pk[i + h] = pack_bf16x2(x, y);
+            }
+          }
+          tmem_st16(tp + c * 16, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&ctl->ds_ready[c]);
+            if (c == 1) mbar_arrive(&ctl->stat_empty[sst]);
           }
         }
       }
-    } else if (n_iter == 0 && kj < g.Sk) {
-      // no query sees these keys: zero gradients (each warp half clears its own 64 columns)
-      if (g.hs > 1) {
-        for (int i = c_lo * 8; i < c_lo * 8 + 16; ++i) {
-          reinterpret_cast<float4*>(pdv)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          reinterpret_cast<float4*>(pdk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      } else {
-        __nv_bfloat16* dvr = dv + (long long)kj * g.dv_s + (long long)b * g.dv_b + (long long)hk * g.dv_h;
-        __nv_bfloat16* dkr = dk + (long long)kj * g.dk_s + (long long)b * g.dk_b + (long long)hk * g.dk_h;
-        for (int i = c_lo * 4; i < c_lo * 4 + 8; ++i) {
-          reinterpret_cast<uint4*>(dvr)[i] = make_uint4(0, 0, 0, 0);
-          reinterpret_cast<uint4*>(dkr)[i] = make_uint4(0, 0, 0, 0);
+      if (++head == gpp) { head = 0; ++qb; }
+    }
+    // epilogue: this thread's key row of dV and of dK (times scale), columns [64 half, 64 half + 64)
+    const long long part_elems = (long long)g.Tk * g.B * g.Hk * D;
+    const long long krow = w.k0 + kj;
+    float* pdv = a.hs > 1 ? a.part + (long long)hpart * part_elems + ((krow * g.B + w.b) * g.Hk + hk) * D + half * 64 : nullptr;
+    float* pdk = a.hs > 1 ? pdv + (long long)a.hs * part_elems : nullptr;
+    __nv_bfloat16* dvr = a.dv + krow * a.dv_s + (long long)w.b * a.dv_b + (long long)hk * a.dv_h + half * 64;
+    __nv_bfloat16* dkr = a.dk + krow * a.dk_s + (long long)w.b * a.dk_b + (long long)hk * a.dk_h + half * 64;
+    if (n_iter > 0) {
+      if (ok && mbar_wait(&ctl->acc_full, 0, abort_flag, g.status, 523)) {
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          uint32_t x[32], y[32];
+          tmem_ld32(tmem + 256 + lane_base + half * 64 + c * 32, x);      // warp-collective: no per-lane branch around it
+          tmem_ld32(tmem + 384 + lane_base + half * 64 + c * 32, y);
+          tmem_ld_wait();
+          if (kj < w.nk) store_dkv_cols(a, g.scale, x, y, pdv + c * 32, pdk + c * 32, dvr + c * 32, dkr + c * 32);
         }
       }
+    } else if (kj < w.nk) {
+      // no query sees these keys: zero gradients
+      uint32_t z[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) z[i] = 0;
+      for (int c = 0; c < 2; ++c) store_dkv_cols(a, g.scale, z, z, pdv + c * 32, pdk + c * 32, dvr + c * 32, dkr + c * 32);
     }
   }
   tc_fence_before();
@@ -896,58 +847,54 @@ __global__ void __launch_bounds__(256) attn_dkv_reduce_kernel(const float* __res
                                                  pack_bf16x2(acc[6], acc[7]));
 }
 
-// ----------------------------------------------------------------------- backward, dQ
-// One CTA per (128 query rows, batch, query head); it loops over the key blocks these
-// queries see, recomputes S = Q K^T and dP = dO V^T, forms dS = P (dP - delta) and
-// accumulates dQ += dS K in TMEM over the whole loop, so that no atomics and no fp32 scratch
-// are needed for dQ (two extra MMAs per tile pair buy that).
+// ----------------------------------------------------------------------- dQ
+constexpr int DQ_KRING = 3, DQ_VRING = 2;
 struct DqCtl {
-  uint64_t qdo_full;
-  uint64_t kv_full[2], kv_empty[2];
-  uint64_t sdp_full, ds_ready, dq_full;
+  uint64_t q_full, do_full;
+  uint64_t k_full[DQ_KRING], k_empty[DQ_KRING], v_full[DQ_VRING], v_empty[DQ_VRING];
+  uint64_t s_full[2], dp_full, ds_ready, dq_full;
   uint32_t tmem_base;
   int abort_flag;
 };
-constexpr int DQ_SMEM = TILE_BYTES * 7 + 1024 + 256;    // Q, dO, K x2, V x2, dS
+constexpr int DQ_SMEM = TILE_BYTES * (2 + DQ_KRING + DQ_VRING) + 1024 + 512;    // Q, dO, K x3, V x2
 
-struct DqGeometry {
-  int B, Hq, Hk, Sq, Sk, causal;
-  float scale;
+struct DqArgs {
+  const float* lse;
+  const float* delta;
+  __nv_bfloat16* dq;
   long long dq_s, dq_b, dq_h;
-  DeviceStatus* status;
-  int x0, p0, ny;                 // as in Geometry; ny = Hq
 };
 
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+template <class Table>
+__global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                   const __grid_constant__ CUtensorMap tdo, const float* __restrict__ lse, const float* __restrict__ delta,
-                   __nv_bfloat16* __restrict__ dq, const DqGeometry g) {
+                   const __grid_constant__ CUtensorMap tdo, const __grid_constant__ Geometry g, const __grid_constant__ DqArgs a,
+                   const __grid_constant__ Table table) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sDO = smem + TILE_BYTES;
   uint8_t* sK = smem + 2 * TILE_BYTES;
-  uint8_t* sV = smem + 4 * TILE_BYTES;
-  uint8_t* sDS = smem + 6 * TILE_BYTES;
-  DqCtl* ctl = reinterpret_cast<DqCtl*>(smem + 7 * TILE_BYTES);
+  uint8_t* sV = smem + (2 + DQ_KRING) * TILE_BYTES;
+  DqCtl* ctl = reinterpret_cast<DqCtl*>(smem + (2 + DQ_KRING + DQ_VRING) * TILE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqb = (g.Sq + BQ - 1) / BQ;
-  const int qb = nqb - 1 - (g.x0 + (int)blockIdx.x);
-  const int pyz = g.p0 + (int)blockIdx.y + (int)blockIdx.z * (int)gridDim.y;
-  const int hq = pyz % g.ny, b = pyz / g.ny;
-  const int hk = hq / (g.Hq / g.Hk);
-  const int off = g.Sk - g.Sq;
-  int nblk = (g.Sk + BKV - 1) / BKV;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const Work w = find_work(g, table, g.x0 + (int)blockIdx.x);
+  const int hq = w.head, hk = hq / (g.Hq / g.Hk);
+  const int qb = sizeof(Table) > 1 ? w.tile : (w.nq + BQ - 1) / BQ - 1 - w.tile;      // dense: latest queries first
+  const int off = w.nk - w.nq;
+  int nblk = (w.nk + BKV - 1) / BKV;
   if (g.causal) {
-    const int last_key = qb * BQ + BQ - 1 + off;
+    const int last_key = min(qb * BQ + BQ, w.nq) - 1 + off;
     nblk = last_key < 0 ? 0 : min(nblk, last_key / BKV + 1);
   }
 
   if (threadIdx.x == 0) {
-    mbar_init(&ctl->qdo_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&ctl->kv_full[i], 1); mbar_init(&ctl->kv_empty[i], 1); }
-    mbar_init(&ctl->sdp_full, 1); mbar_init(&ctl->ds_ready, 8); mbar_init(&ctl->dq_full, 1);
+    mbar_init(&ctl->q_full, 1); mbar_init(&ctl->do_full, 1);
+    for (int i = 0; i < DQ_KRING; ++i) { mbar_init(&ctl->k_full[i], 1); mbar_init(&ctl->k_empty[i], 1); }
+    for (int i = 0; i < DQ_VRING; ++i) { mbar_init(&ctl->v_full[i], 1); mbar_init(&ctl->v_empty[i], 1); }
+    mbar_init(&ctl->s_full[0], 1); mbar_init(&ctl->s_full[1], 1);
+    mbar_init(&ctl->dp_full, 1); mbar_init(&ctl->ds_ready, 8); mbar_init(&ctl->dq_full, 1);
     ctl->abort_flag = 0;
     mbar_fence_init();
   }
@@ -955,124 +902,176 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort_flag;
-  // TMEM columns: [0,128) S, [128,256) dP, [256,384) dQ
+  // TMEM columns: S [0,128) and [128,256) in turn, dP [256,384) overwritten by its bf16 dS, dQ [384,512)
 
   if (warp == 0) {
     if (lane == 0 && nblk > 0) {
       tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv); tma_prefetch_desc(&tdo);
-      mbar_expect_tx(&ctl->qdo_full, 2 * TILE_BYTES);
-      tma_load_4d(sQ, &tq, &ctl->qdo_full, 0, hq, b, qb * BQ);
-      tma_load_4d(sQ + HALF_BYTES, &tq, &ctl->qdo_full, 64, hq, b, qb * BQ);
-      tma_load_4d(sDO, &tdo, &ctl->qdo_full, 0, hq, b, qb * BQ);
-      tma_load_4d(sDO + HALF_BYTES, &tdo, &ctl->qdo_full, 64, hq, b, qb * BQ);
+      mbar_expect_tx(&ctl->q_full, TILE_BYTES);
+      load_tile(sQ, &tq, &ctl->q_full, hq, w.b, w.q0 + qb * BQ);
+      int ks = 0, vs = 0;
+      uint32_t kph = 1, vph = 1;
       for (int j = 0; j < nblk; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&ctl->kv_empty[s], ((j >> 1) & 1) ^ 1, abort_flag, g.status, 800)) break;
-        mbar_expect_tx(&ctl->kv_full[s], 2 * TILE_BYTES);
-        tma_load_4d(sK + s * TILE_BYTES, &tk, &ctl->kv_full[s], 0, hk, b, j * BKV);
-        tma_load_4d(sK + s * TILE_BYTES + HALF_BYTES, &tk, &ctl->kv_full[s], 64, hk, b, j * BKV);
-        tma_load_4d(sV + s * TILE_BYTES, &tv, &ctl->kv_full[s], 0, hk, b, j * BKV);
-        tma_load_4d(sV + s * TILE_BYTES + HALF_BYTES, &tv, &ctl->kv_full[s], 64, hk, b, j * BKV);
+        if (!mbar_wait(&ctl->k_empty[ks], kph, abort_flag, g.status, 800)) break;
+        mbar_expect_tx(&ctl->k_full[ks], TILE_BYTES);
+        load_tile(sK + ks * TILE_BYTES, &tk, &ctl->k_full[ks], hk, w.b, w.k0 + j * BKV);
+        if (j == 0) {
+          mbar_expect_tx(&ctl->do_full, TILE_BYTES);
+          load_tile(sDO, &tdo, &ctl->do_full, hq, w.b, w.q0 + qb * BQ);
+        }
+        if (!mbar_wait(&ctl->v_empty[vs], vph, abort_flag, g.status, 801)) break;
+        mbar_expect_tx(&ctl->v_full[vs], TILE_BYTES);
+        load_tile(sV + vs * TILE_BYTES, &tv, &ctl->v_full[vs], hk, w.b, w.k0 + j * BKV);
+        if (++ks == DQ_KRING) { ks = 0; kph ^= 1; }
+        if (++vs == DQ_VRING) { vs = 0; vph ^= 1; }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && nblk > 0) {
+    const uint32_t leader = elect_one();
+    if (nblk > 0) {
       constexpr uint32_t id_kk = umma_idesc_bf16(128, 128, 0, 0);   // S, dP
-      constexpr uint32_t id_km = umma_idesc_bf16(128, 128, 0, 1);   // dQ: dS K-major, K MN-major
-      const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO), ds_base = smem_u32(sDS);
-      bool ok = mbar_wait(&ctl->qdo_full, 0, abort_flag, g.status, 810);
+      constexpr uint32_t id_km = umma_idesc_bf16(128, 128, 0, 1);   // dQ: A = dS in TMEM, B = K MN-major
+      const uint32_t q_base = smem_u32(sQ), do_base = smem_u32(sDO);
+      int kslot = 0, vslot = 0;                        // ring slots of the NEXT K (S product) and V (dP product)
+      uint32_t kph = 0, vph = 0;
+      auto issue_s = [&](int j) -> bool {
+        if (!warp_wait(&ctl->k_full[kslot], kph, abort_flag, g.status, 811)) return false;
+        tc_fence_after();
+        {
+          const uint32_t k_base = smem_u32(sK + kslot * TILE_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) umma_bf16_by(leader, tmem + (j & 1) * 128, desc_kmajor(q_base, kk), desc_kmajor(k_base, kk), id_kk, kk > 0);
+          umma_commit_by(leader, &ctl->s_full[j & 1]);
+        }
+        if (++kslot == DQ_KRING) { kslot = 0; kph ^= 1; }
+        return true;
+      };
+      auto issue_dp = [&]() -> bool {
+        if (!warp_wait(&ctl->v_full[vslot], vph, abort_flag, g.status, 812)) return false;
+        tc_fence_after();
+        {
+          const uint32_t v_base = smem_u32(sV + vslot * TILE_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) umma_bf16_by(leader, tmem + 256, desc_kmajor(do_base, kk), desc_kmajor(v_base, kk), id_kk, kk > 0);
+          umma_commit_by(leader, &ctl->dp_full);
+          umma_commit_by(leader, &ctl->v_empty[vslot]);
+        }
+        if (++vslot == DQ_VRING) { vslot = 0; vph ^= 1; }
+        return true;
+      };
+      bool ok = warp_wait(&ctl->q_full, 0, abort_flag, g.status, 810) && issue_s(0) &&
+                warp_wait(&ctl->do_full, 0, abort_flag, g.status, 810) && issue_dp();
+      int dslot = 0;                                   // ring slot of K_j for the dQ product
       for (int j = 0; j < nblk && ok; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&ctl->kv_full[s], (j >> 1) & 1, abort_flag, g.status, 811)) break;
+        // the other S buffer was read before dS(j-1) was announced
+        if (j + 1 < nblk && !issue_s(j + 1)) { ok = false; break; }
+        if (!warp_wait(&ctl->ds_ready, j & 1, abort_flag, g.status, 813)) { ok = false; break; }
+        if (sizeof(Table) > 1 && (j + 1) * BKV > w.nk && w.k0 + w.nk < g.Tk) zero_tile_rows(sK + dslot * TILE_BYTES, w.nk - j * BKV, lane);
         tc_fence_after();
-        const uint32_t k_base = smem_u32(sK + s * TILE_BYTES), v_base = smem_u32(sV + s * TILE_BYTES);
+        {
+          const uint32_t k_base = smem_u32(sK + dslot * TILE_BYTES);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 0, desc_kmajor(q_base, kk), desc_kmajor(k_base, kk), id_kk, kk > 0);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 128, desc_kmajor(do_base, kk), desc_kmajor(v_base, kk), id_kk, kk > 0);
-        umma_commit(&ctl->sdp_full);
-        if (!mbar_wait(&ctl->ds_ready, j & 1, abort_flag, g.status, 812)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 256, desc_kmajor(ds_base, kk), desc_mnmajor(k_base, kk), id_km, (j | kk) != 0);
-        umma_commit(&ctl->kv_empty[s]);
+          for (int kk = 0; kk < 8; ++kk)
+            umma_bf16_ts_by(leader, tmem + 384, tmem + 256 + (kk >> 2) * 64 + (kk & 3) * 8, desc_mnmajor(k_base, kk), id_km, (j | kk) != 0);
+          umma_commit_by(leader, &ctl->k_empty[dslot]);
+        }
+        if (++dslot == DQ_KRING) dslot = 0;
+        if (j + 1 < nblk && !issue_dp()) { ok = false; break; }     // in order behind the product that reads dS
       }
-      if (ok) umma_commit(&ctl->dq_full);
+      if (ok) umma_commit_by(leader, &ctl->dq_full);
     }
     __syncwarp();
-  } else {
+  } else if (warp >= MATH_WARP0) {
     const int quarter = warp & 3;
-    const int c_lo = ((warp - 2) >> 2) * 2;
-    const int r = quarter * 32 + lane;
-    const int qi = qb * BQ + r;
-    const bool row_ok = qi < g.Sq;
+    const int half = (warp - MATH_WARP0) >> 2;         // key columns [64 half, 64 half + 64)
+    const int qi = qb * BQ + quarter * 32 + lane;
+    const bool row_ok = qi < w.nq;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t ts = tmem + lane_base + half * 64, tp = ts + 256;
     const float sl2 = g.scale * LOG2E;
-    const long long stat = ((long long)b * g.Hq + hq) * g.Sq + qi;
-    const float L = row_ok ? lse[stat] * LOG2E : 0.f;
-    const float dl = row_ok ? delta[stat] : 0.f;
+    const uint64_t sl2_2 = pk2(sl2, sl2);
+    const float nL = row_ok ? -a.lse[((long long)w.sid * g.Hq + hq) * g.ls + qi] * LOG2E : -INFINITY;
+    const float nD = row_ok ? -a.delta[((long long)w.b * g.Hq + hq) * g.Tq + w.q0 + qi] : 0.f;
+    const uint64_t nL2 = pk2(nL, nL), nD2 = pk2(nD, nD);
     bool ok = nblk > 0;
     for (int j = 0; j < nblk && ok; ++j) {
-      if (!mbar_wait(&ctl->sdp_full, j & 1, abort_flag, g.status, 820)) { ok = false; break; }
-      tc_fence_after();
-      const int key0 = j * BKV;
-      int limit = g.Sk - key0;
-      if (g.causal) limit = min(limit, qi + off - key0 + 1);
+      int limit = visible_keys(w.nk, g.causal, off, qi, j * BKV + half * 64);
       if (!row_ok) limit = 0;
-#pragma unroll 1
-      for (int c = c_lo; c < c_lo + 2; ++c) {
-        uint32_t sv[32], dpv[32];
-        tmem_ld32(tmem + 0 + lane_base + c * 32, sv);
-        tmem_ld32(tmem + 128 + lane_base + c * 32, dpv);
-        tmem_ld_wait();
+      const bool full = __all_sync(0xffffffffu, limit >= 64);
+      if (!mbar_wait(&ctl->s_full[j & 1], (j >> 1) & 1, abort_flag, g.status, 820)) { ok = false; break; }
+      tc_fence_after();
+      auto gradients = [&](auto edge_) -> bool {       // as in the dK/dV kernel, the mask is a path of its own
+        constexpr bool masked = decltype(edge_)::value;
+        uint64_t p[32];
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          float ds[8];
+        for (int c = 0; c < 2; ++c) {
+          uint32_t s[32];
+          tmem_ld32(ts + (j & 1) * 128 + c * 32, s);
+          tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int col = c * 32 + q4 * 8 + i;
-            float pe = exp2f(__uint_as_float(sv[q4 * 8 + i]) * sl2 - L);
-            if (col >= limit) pe = 0.f;
-            ds[i] = pe * (__uint_as_float(dpv[q4 * 8 + i]) - dl);
+          for (int i = 0; i < 16; ++i) {
+            float x, y;
+            upk2(fma2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sl2_2, nL2), x, y);
+            p[c * 16 + i] = pk2(ex2(x), ex2(y));
           }
-          uint4 ud;
-          ud.x = pack_bf16x2(ds[0], ds[1]); ud.y = pack_bf16x2(ds[2], ds[3]); ud.z = pack_bf16x2(ds[4], ds[5]); ud.w = pack_bf16x2(ds[6], ds[7]);
-          *reinterpret_cast<uint4*>(sDS + swz_off(r, c * 4 + q4)) = ud;
         }
-      }
+        if (!mbar_wait(&ctl->dp_full, j & 1, abort_flag, g.status, 821)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tp + c * 32, v);
+          tmem_ld_wait();
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float x, y;
+            upk2(mul2(p[c * 16 + i], add2(pk2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), nD2)), x, y);
+            if (masked) {                              // whatever a masked key or a neighbour's row has left in S or dP
+              if (c * 32 + 2 * i >= limit) x = 0.f;
+              if (c * 32 + 2 * i + 1 >= limit) y = 0.f;
+            }
+            pk[i] = pack_bf16x2(x, y);
+          }
+          tmem_st16(tp + c * 16, pk);
+        }
+        return true;
+      };
+      ok = full ? gradients(std::false_type{}) : gradients(std::true_type{});
+      if (!ok) break;
+      tmem_st_wait();
       tc_fence_before();
-      fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->ds_ready);
     }
-    __nv_bfloat16* dqr = dq + (long long)qi * g.dq_s + (long long)b * g.dq_b + (long long)hq * g.dq_h;
-    if (ok && nblk > 0) {
-      if (mbar_wait(&ctl->dq_full, 0, abort_flag, g.status, 821)) {
+    __nv_bfloat16* dqr = a.dq + (long long)(w.q0 + qi) * a.dq_s + (long long)w.b * a.dq_b + (long long)hq * a.dq_h + half * 64;
+    if (nblk > 0) {
+      if (ok && mbar_wait(&ctl->dq_full, 0, abort_flag, g.status, 822)) {
         tc_fence_after();
 #pragma unroll 1
-        for (int c = c_lo; c < c_lo + 2; ++c) {
-          uint32_t a[32];
-          tmem_ld32(tmem + 256 + lane_base + c * 32, a);
+        for (int c = 0; c < 2; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tmem + 384 + lane_base + half * 64 + c * 32, v);
           tmem_ld_wait();
           if (row_ok) {
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
               uint4 u;
               const int i0 = q4 * 8;
-              u.x = pack_bf16x2(__uint_as_float(a[i0]) * g.scale, __uint_as_float(a[i0 + 1]) * g.scale);
-              u.y = pack_bf16x2(__uint_as_float(a[i0 + 2]) * g.scale, __uint_as_float(a[i0 + 3]) * g.scale);
-              u.z = pack_bf16x2(__uint_as_float(a[i0 + 4]) * g.scale, __uint_as_float(a[i0 + 5]) * g.scale);
-              u.w = pack_bf16x2(__uint_as_float(a[i0 + 6]) * g.scale, __uint_as_float(a[i0 + 7]) * g.scale);
+              u.x = pack_bf16x2(__uint_as_float(v[i0]) * g.scale, __uint_as_float(v[i0 + 1]) * g.scale);
+              u.y = pack_bf16x2(__uint_as_float(v[i0 + 2]) * g.scale, __uint_as_float(v[i0 + 3]) * g.scale);
+              u.z = pack_bf16x2(__uint_as_float(v[i0 + 4]) * g.scale, __uint_as_float(v[i0 + 5]) * g.scale);
+              u.w = pack_bf16x2(__uint_as_float(v[i0 + 6]) * g.scale, __uint_as_float(v[i0 + 7]) * g.scale);
               reinterpret_cast<uint4*>(dqr + c * 32)[q4] = u;
             }
           }
         }
       }
-    } else if (nblk == 0 && row_ok && c_lo == 0) {
-      for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(dqr)[i] = make_uint4(0, 0, 0, 0);
+    } else if (row_ok) {
+      for (int i = 0; i < 8; ++i) reinterpret_cast<uint4*>(dqr)[i] = make_uint4(0, 0, 0, 0);
     }
   }
   tc_fence_before();
@@ -1080,13 +1079,231 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-
-static const CUtensorMap* tensor_map_sbhd(const void* p, int S, int B, int H, long long s_s, long long s_b, long long s_h,
-                                          uint32_t box_rows = 128) {
+static const CUtensorMap* tensor_map_sbhd(const void* p, int S, int B, int H, long long s_s, long long s_b, long long s_h) {
   const uint64_t dims[4] = {(uint64_t)D, (uint64_t)H, (uint64_t)B, (uint64_t)S};
   const uint64_t st[3] = {(uint64_t)s_h * 2, (uint64_t)s_b * 2, (uint64_t)s_s * 2};
-  const uint32_t box[4] = {64, 1, 1, box_rows};
+  const uint32_t box[4] = {64, 1, 1, 128};
   return get_tmap_4d(p, 2, dims, st, box, true);
+}
+
+// Shared-memory opt-in, once per kernel and device.
+template <class Kernel>
+static cudaError_t opt_in(Kernel kern, int bytes, PerDeviceFlags& done_on) {
+  bool& done = device_flag(done_on);
+  if (done) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) set_last_error("attention: shared memory opt-in failed: %s", cudaGetErrorString(e));
+  else done = true;
+  return e;
+}
+
+// SM budget for kernels whose grid is one CTA per work item (one CTA per SM by shared memory): the items are cut into
+// launches of at most `budget` CTAs, which the stream runs one after the other, so at most `budget` SMs are in use at
+// any time.  launch(count, x0) starts items x0 .. x0 + count - 1.
+template <class F>
+static void launch_in_waves(long long items, int sm_budget, F&& launch) {
+  const int sms = dh_sm_count();
+  const long long wave = (sm_budget <= 0 || sm_budget >= sms) ? items : sm_budget;
+  for (long long x0 = 0; x0 < items; x0 += wave) launch((unsigned)std::min(wave, items - x0), (int)x0);
+}
+
+// Tiles of a packed batch in descending order of work, cut into launches that fit one kernel parameter.
+// work(nq, nk, tile) = key (query) blocks of that tile; rows(nq, nk) = what the tiles cover, `per` rows each.
+struct Sequences {
+  int n;
+  const int* cu_q;
+  const int* cu_k;
+};
+template <class Rows, class Cost, class F>
+static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows, Cost&& cost, F&& launch) {
+  struct T { long long cost; int seq, tile; };
+  std::vector<T> tiles;
+  for (int s = 0; s < sq.n; ++s) {
+    const int nq = sq.cu_q[s + 1] - sq.cu_q[s], nk = sq.cu_k[s + 1] - sq.cu_k[s];
+    const int n = (rows(nq, nk) + per - 1) / per;
+    if (n > 65536) { set_last_error("attention: a sequence of %d rows is longer than a packed batch supports", rows(nq, nk)); return cudaErrorInvalidValue; }
+    for (int t = 0; t < n; ++t) tiles.push_back({cost(nq, nk, t), s, t});
+  }
+  std::stable_sort(tiles.begin(), tiles.end(), [](const T& a, const T& b) { return a.cost > b.cost; });
+  std::vector<int> slot(sq.n, -1);
+  Packed p;
+  int ns = 0, nt = 0;
+  auto flush = [&]() {
+    if (nt == 0) return;
+    launch(p, nt);
+    for (int i = 0; i < ns; ++i) slot[p.id[i]] = -1;
+    ns = nt = 0;
+  };
+  for (const T& t : tiles) {
+    if (nt == MAX_TILES || (slot[t.seq] < 0 && ns == MAX_SEQS)) flush();
+    if (slot[t.seq] < 0) {
+      slot[t.seq] = ns;
+      p.q0[ns] = sq.cu_q[t.seq]; p.nq[ns] = sq.cu_q[t.seq + 1] - sq.cu_q[t.seq];
+      p.k0[ns] = sq.cu_k[t.seq]; p.nk[ns] = sq.cu_k[t.seq + 1] - sq.cu_k[t.seq];
+      p.id[ns++] = t.seq;
+    }
+    p.tile[nt++] = (uint32_t)slot[t.seq] << 16 | (uint32_t)t.tile;
+  }
+  flush();
+  return cudaSuccess;
+}
+static bool offsets_ok(const char* who, const Sequences& s, int Tq, int Tk, int max_q) {
+  for (int i = 0; i < s.n; ++i) {
+    const int nq = s.cu_q[i + 1] - s.cu_q[i], nk = s.cu_k[i + 1] - s.cu_k[i];
+    if (s.cu_q[i] < 0 || s.cu_k[i] < 0 || nq < 0 || nk < 0 || nq > max_q || s.cu_q[i + 1] > Tq || s.cu_k[i + 1] > Tk) {
+      set_last_error("%s: sequence %d (queries %d..%d, keys %d..%d) does not fit the packed tensors or the longest length %d", who, i,
+                     s.cu_q[i], s.cu_q[i + 1], s.cu_k[i], s.cu_k[i + 1], max_q);
+      return false;
+    }
+  }
+  return true;
+}
+// Key blocks that query rows [first, first + rows) see / query blocks that see a key block.
+static long long key_blocks(int nq, int nk, int causal, int first, int rows) {
+  long long n = (nk + BKV - 1) / BKV;
+  if (causal) {
+    const long long last_key = (long long)std::min(first + rows, nq) - 1 + nk - nq;
+    n = last_key < 0 ? 0 : std::min(n, last_key / BKV + 1);
+  }
+  return n;
+}
+static long long query_blocks(int nq, int nk, int causal, int kb) {
+  const long long n = (nq + BQ - 1) / BQ;
+  const long long first_q = causal ? (long long)kb * BKV - (nk - nq) : 0;
+  return std::max(0ll, n - (first_q <= 0 ? 0 : first_q / BQ));
+}
+
+struct FwdMaps { const CUtensorMap *q, *k, *v; };
+template <class Table>
+static void run_fwd(const FwdMaps& m, Geometry& g, const FwdArgs& a, const Table& table, long long items, int sm_budget, cudaStream_t stream) {
+  launch_in_waves(items, sm_budget, [&](unsigned n, int x0) {
+    g.x0 = x0;
+    attn_fwd_kernel<Table><<<n, THREADS, FWD_SMEM, stream>>>(*m.q, *m.k, *m.v, g, a, table);
+  });
+}
+
+// Two query heads of a KV group per CTA where groups are even: both tiles then see the same keys whatever the mask, and
+// a sequence of up to 128 rows fills the CTA.  Odd groups (one query head per KV head) take two row tiles instead.
+static int fwd_head_pair(int Hq, int Hk) { return (Hq / Hk) % 2 == 0; }
+
+// Number of CTAs that share the query heads of one KV head in the dK/dV kernel: 1 while
+// KV blocks x batch x KV heads already give every SM a few CTAs, else the smallest power of
+// two (dividing the group size) that does.
+static int bwd_head_split(long long kv_tiles, int Hq, int Hk) {
+  static int enabled = -1;
+  if (enabled < 0) {
+    const char* e = getenv("DHELLAM_ATTN_HEAD_SPLIT");
+    enabled = e ? atoi(e) : 1;
+  }
+  if (!enabled) return 1;
+  const int group = Hq / Hk;
+  const long long ctas = kv_tiles * Hk;
+  int hs = 1;
+  while (hs < group && group % (hs * 2) == 0 && ctas * hs < 4LL * dh_sm_count()) hs *= 2;
+  return hs;
+}
+static long long packed_kv_tiles(int nseq, const int* cu_k) {
+  long long n = 0;
+  for (int s = 0; s < nseq; ++s) n += (cu_k[s + 1] - cu_k[s] + BKV - 1) / BKV;
+  return n;
+}
+// Scratch of the backward: delta [B*Hq*Tq] fp32 (row dot products of dO and O), rounded up to 256 bytes, then, when
+// the dK/dV kernel splits heads, the fp32 partials [2][hs][Tk][B][Hk][128].
+static int64_t delta_bytes(int B, int Hq, int Tq) { return ((int64_t)B * Hq * Tq * 4 + 255) / 256 * 256; }
+static int64_t scratch_bytes(int B, int Hq, int Hk, int Tq, int Tk, int hs) {
+  return delta_bytes(B, Hq, Tq) + (hs > 1 ? (int64_t)2 * hs * Tk * B * Hk * D * 4 : 0);
+}
+
+static void launch_delta(const void* dout, const void* out, float* delta, int B, int Hq, int T, const int64_t* sdo, const int64_t* so,
+                         cudaStream_t stream) {
+  // dO is a TMA operand (16-byte aligned throughout); O need not be
+  const int wide = ((reinterpret_cast<uintptr_t>(out) | (uintptr_t)(so[0] * 2) | (uintptr_t)(so[1] * 2) | (uintptr_t)(so[2] * 2)) & 15) == 0;
+  attn_delta_kernel<<<dim3((unsigned)((T + 63) / 64 * Hq), B), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, Hq, T,
+                                                                                 sdo[0], sdo[1], sdo[2], so[0], so[1], so[2], wide);
+}
+
+struct BwdMaps { const CUtensorMap *q, *k, *v, *dout; };
+template <class Table>
+static void run_dkv(const BwdMaps& m, Geometry& g, const DkvArgs& a, const Table& table, long long items, int sm_budget, cudaStream_t stream) {
+  g.heads = g.Hk * a.hs;
+  launch_in_waves(items, sm_budget, [&](unsigned n, int x0) {
+    g.x0 = x0;
+    attn_bwd_dkv_kernel<Table><<<n, THREADS, DKV_SMEM, stream>>>(*m.q, *m.k, *m.v, *m.dout, g, a, table);
+  });
+}
+template <class Table>
+static void run_dq(const BwdMaps& m, Geometry& g, const DqArgs& a, const Table& table, long long items, int sm_budget, cudaStream_t stream) {
+  g.heads = g.Hq;
+  launch_in_waves(items, sm_budget, [&](unsigned n, int x0) {
+    g.x0 = x0;
+    attn_bwd_dq_kernel<Table><<<n, THREADS, DQ_SMEM, stream>>>(*m.q, *m.k, *m.v, *m.dout, g, a, table);
+  });
+}
+template <class Table>
+static cudaError_t opt_in_fwd() {
+  static PerDeviceFlags done;
+  return opt_in(attn_fwd_kernel<Table>, FWD_SMEM, done);
+}
+template <class Table>
+static cudaError_t opt_in_bwd() {
+  static PerDeviceFlags done_kv, done_q;
+  cudaError_t e = opt_in(attn_bwd_dkv_kernel<Table>, DKV_SMEM, done_kv);
+  return e != cudaSuccess ? e : opt_in(attn_bwd_dq_kernel<Table>, DQ_SMEM, done_q);
+}
+
+// One backward over either kind of batch; `seqs` null = dense.
+static int bwd_common(const void* dout, const void* out, const void* lse, void* dq, void* dk, void* dv, void* scratch, const int64_t* strides,
+                      const BwdMaps& maps, Geometry g, int hs, const Sequences* seqs, int sm_budget, cudaStream_t stream) {
+  const int64_t* sdo = strides; const int64_t* so = strides + 12;
+  const int64_t* sdq = strides + 15; const int64_t* sdk = strides + 18; const int64_t* sdv = strides + 21;
+  float* delta = reinterpret_cast<float*>(scratch);
+  launch_delta(dout, out, delta, g.B, g.Hq, g.Tq, sdo, so, stream);
+  DkvArgs a;
+  a.lse = (const float*)lse; a.delta = delta;
+  a.dk = (__nv_bfloat16*)dk; a.dv = (__nv_bfloat16*)dv;
+  a.dk_s = sdk[0]; a.dk_b = sdk[1]; a.dk_h = sdk[2]; a.dv_s = sdv[0]; a.dv_b = sdv[1]; a.dv_h = sdv[2];
+  a.hs = hs;
+  a.part = hs > 1 ? reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + delta_bytes(g.B, g.Hq, g.Tq)) : nullptr;
+  DqArgs aq;
+  aq.lse = (const float*)lse; aq.delta = delta; aq.dq = (__nv_bfloat16*)dq;
+  aq.dq_s = sdq[0]; aq.dq_b = sdq[1]; aq.dq_h = sdq[2];
+  cudaError_t e = cudaSuccess;
+  if (seqs == nullptr) {
+    run_dkv(maps, g, a, Dense{}, (long long)((g.Sk + BKV - 1) / BKV) * g.B * g.Hk * hs, sm_budget, stream);
+  } else {
+    e = for_packed_launches(*seqs, BKV, [](int, int nk) { return nk; }, [&](int nq, int nk, int t) { return query_blocks(nq, nk, g.causal, t); },
+                            [&](const Packed& p, int n) { run_dkv(maps, g, a, p, (long long)n * g.Hk * hs, sm_budget, stream); });
+    if (e != cudaSuccess) return (int)e;
+  }
+  if (hs > 1) {
+    const long long n = 2LL * g.Tk * g.B * g.Hk * (D / 8);
+    attn_dkv_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(a.part, hs, a.dk, a.dv, g.Tk, g.B, g.Hk, sdk[0], sdk[1], sdk[2],
+                                                                           sdv[0], sdv[1], sdv[2]);
+  }
+  if (seqs == nullptr) {
+    run_dq(maps, g, aq, Dense{}, (long long)((g.Sq + BQ - 1) / BQ) * g.B * g.Hq, sm_budget, stream);
+  } else {
+    e = for_packed_launches(*seqs, BQ, [](int nq, int) { return nq; },
+                            [&](int nq, int nk, int t) { return key_blocks(nq, nk, g.causal, t * BQ, BQ); },
+                            [&](const Packed& p, int n) { run_dq(maps, g, aq, p, (long long)n * g.Hq, sm_budget, stream); });
+    if (e != cudaSuccess) return (int)e;
+  }
+  e = cudaGetLastError();
+  if (e != cudaSuccess) set_last_error("attention backward launch failed: %s", cudaGetErrorString(e));
+  return (int)e;
+}
+
+static Geometry geometry(int B, int Hq, int Hk, int Sq, int Sk, int Tq, int Tk, int ls, int causal, float scale) {
+  Geometry g;
+  g.B = B; g.Hq = Hq; g.Hk = Hk; g.Sq = Sq; g.Sk = Sk; g.Tq = Tq; g.Tk = Tk; g.ls = ls; g.causal = causal; g.scale = scale;
+  g.x0 = 0; g.heads = Hq;
+  g.status = reinterpret_cast<DeviceStatus*>(dh_status_device_ptr());
+  return g;
+}
+static bool heads_ok(const char* who, int d, int Hq, int Hk) {
+  if (d != D) { set_last_error("%s: head size %d is not supported (128 only)", who, d); return false; }
+  if (Hk <= 0 || Hq % Hk != 0) { set_last_error("%s: query heads must be a multiple of KV heads", who); return false; }
+  return true;
 }
 
 }  // namespace attn
@@ -1095,176 +1312,115 @@ static const CUtensorMap* tensor_map_sbhd(const void* p, int S, int B, int H, lo
 using namespace dh;
 using namespace dh::attn;
 
-// dK/dV kernel choice of dh_attn_bwd: -1 = read DHELLAM_ATTN_BWD_T on first use, 0 = attn_bwd_kernel, 1 = attn_bwd_t_kernel
-static int g_bwd_mode = -1;
-
-// SM budget for kernels whose grid is one CTA per tile (one CTA per SM by shared memory): the (X, Y, Z) grid is cut
-// into launches of at most `budget` CTAs, which the stream runs one after the other, so at most `budget` SMs are in
-// use at any time.  launch(grid, x0, p0) starts tile columns x0.. and flattened (y, z) pairs p0..
-template <class F>
-static void launch_in_waves(int X, int Y, int Z, int sm_budget, F&& launch) {
-  const int sms = dh_sm_count();
-  const int budget = (sm_budget <= 0 || sm_budget >= sms) ? 0 : sm_budget;
-  const long long pairs = (long long)Y * Z;
-  if (budget == 0 || (long long)X * pairs <= budget) {
-    launch(dim3(X, Y, Z), 0, 0);
-    return;
-  }
-  if (X >= budget) {
-    for (long long p = 0; p < pairs; ++p)
-      for (int x0 = 0; x0 < X; x0 += budget) launch(dim3(X - x0 < budget ? X - x0 : budget, 1, 1), x0, (int)p);
-  } else {
-    const int np = budget / X;
-    for (long long p0 = 0; p0 < pairs; p0 += np) launch(dim3(X, (unsigned)(pairs - p0 < np ? pairs - p0 : np), 1), 0, (int)p0);
-  }
-}
-
 extern "C" {
 
-void dh_attn_set_bwd_mode(int mode) { g_bwd_mode = mode; }
+// There is one dK/dV kernel; callers that used to choose between two forms are accepted.
+void dh_attn_set_bwd_mode(int) {}
 
 int dh_attn_fwd(const void* q, const void* k, const void* v, void* out, void* lse, int64_t q_s, int64_t q_b, int64_t q_h, int64_t k_s,
                 int64_t k_b, int64_t k_h, int64_t v_s, int64_t v_b, int64_t v_h, int B, int Hq, int Hk, int Sq, int Sk, int d, int causal,
                 float scale, int sm_budget, cudaStream_t stream) {
-  if (d != D) { set_last_error("dh_attn_fwd: head size %d is not supported (128 only)", d); return (int)cudaErrorInvalidValue; }
-  if (Hq % Hk != 0) { set_last_error("dh_attn_fwd: query heads must be a multiple of KV heads"); return (int)cudaErrorInvalidValue; }
+  if (!heads_ok("dh_attn_fwd", d, Hq, Hk)) return (int)cudaErrorInvalidValue;
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  const CUtensorMap* tq = tensor_map_sbhd(q, Sq, B, Hq, q_s, q_b, q_h);
-  const CUtensorMap* tk = tensor_map_sbhd(k, Sk, B, Hk, k_s, k_b, k_h);
-  const CUtensorMap* tv = tensor_map_sbhd(v, Sk, B, Hk, v_s, v_b, v_h);
-  if (!tq || !tk || !tv) return (int)cudaErrorInvalidValue;
-  static PerDeviceFlags configured_on;
-  bool& configured = device_flag(configured_on);
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
-    if (e != cudaSuccess) { set_last_error("dh_attn_fwd: shared memory opt-in failed: %s", cudaGetErrorString(e)); return (int)e; }
-    configured = true;
-  }
-  Geometry g;
-  g.B = B; g.Hq = Hq; g.Hk = Hk; g.Sq = Sq; g.Sk = Sk; g.causal = causal; g.scale = scale;
-  g.o_h = D; g.o_b = (long long)Hq * D; g.o_s = (long long)B * Hq * D;
-  g.status = reinterpret_cast<DeviceStatus*>(dh_status_device_ptr());
-  g.ny = Hq;
-  launch_in_waves((Sq + BQ - 1) / BQ, Hq, B, sm_budget, [&](dim3 grid, int x0, int p0) {
-    g.x0 = x0; g.p0 = p0;
-    attn_fwd_kernel<<<grid, FWD_THREADS, FWD_SMEM, stream>>>(*tq, *tk, *tv, (__nv_bfloat16*)out, (float*)lse, g);
-  });
-  cudaError_t e = cudaGetLastError();
+  const FwdMaps m = {tensor_map_sbhd(q, Sq, B, Hq, q_s, q_b, q_h), tensor_map_sbhd(k, Sk, B, Hk, k_s, k_b, k_h),
+                     tensor_map_sbhd(v, Sk, B, Hk, v_s, v_b, v_h)};
+  if (!m.q || !m.k || !m.v) return (int)cudaErrorInvalidValue;
+  cudaError_t e = opt_in_fwd<Dense>();
+  if (e != cudaSuccess) return (int)e;
+  Geometry g = geometry(B, Hq, Hk, Sq, Sk, Sq, Sk, Sq, causal, scale);
+  FwdArgs a;
+  a.out = (__nv_bfloat16*)out; a.lse = (float*)lse;
+  a.o_h = D; a.o_b = (long long)Hq * D; a.o_s = (long long)B * Hq * D;
+  a.head_pair = fwd_head_pair(Hq, Hk);
+  const int per = a.head_pair ? BQ : 2 * BQ;
+  g.heads = a.head_pair ? Hq / 2 : Hq;
+  run_fwd(m, g, a, Dense{}, (long long)((Sq + per - 1) / per) * g.heads * B, sm_budget, stream);
+  e = cudaGetLastError();
   if (e != cudaSuccess) set_last_error("dh_attn_fwd launch failed: %s", cudaGetErrorString(e));
   return (int)e;
 }
 
-// Number of CTAs that share the query heads of one KV head in the dK/dV kernel: 1 while
-// KV blocks x batch x KV heads already give every SM a few CTAs, else the smallest power of
-// two (dividing the group size) that does.
-static int bwd_head_split(int B, int Hq, int Hk, int Sk) {
-  static int enabled = -1;
-  if (enabled < 0) {
-    const char* e = getenv("DHELLAM_ATTN_HEAD_SPLIT");
-    enabled = e ? atoi(e) : 1;
-  }
-  if (!enabled) return 1;
-  const int group = Hq / Hk;
-  const long long ctas = (long long)((Sk + BKV - 1) / BKV) * B * Hk;
-  int hs = 1;
-  while (hs < group && group % (hs * 2) == 0 && ctas * hs < 4LL * dh_sm_count()) hs *= 2;
-  return hs;
+int dh_attn_fwd_packed(const void* q, const void* k, const void* v, void* out, void* lse, const int64_t* strides /* q,k,v,out x (row,head) */,
+                       int nseq, const int* cu_q, const int* cu_k, int Tq, int Tk, int max_q, int Hq, int Hk, int d, int causal, float scale,
+                       int sm_budget, cudaStream_t stream) {
+  if (!heads_ok("dh_attn_fwd_packed", d, Hq, Hk)) return (int)cudaErrorInvalidValue;
+  if (nseq <= 0 || Tq <= 0 || Tk <= 0) return 0;
+  const Sequences seqs = {nseq, cu_q, cu_k};
+  if (!offsets_ok("dh_attn_fwd_packed", seqs, Tq, Tk, max_q)) return (int)cudaErrorInvalidValue;
+  // the batch dimension has one entry: its stride only has to be a valid one
+  const FwdMaps m = {tensor_map_sbhd(q, Tq, 1, Hq, strides[0], strides[0], strides[1]), tensor_map_sbhd(k, Tk, 1, Hk, strides[2], strides[2], strides[3]),
+                     tensor_map_sbhd(v, Tk, 1, Hk, strides[4], strides[4], strides[5])};
+  if (!m.q || !m.k || !m.v) return (int)cudaErrorInvalidValue;
+  cudaError_t e = opt_in_fwd<Packed>();
+  if (e != cudaSuccess) return (int)e;
+  Geometry g = geometry(1, Hq, Hk, 0, 0, Tq, Tk, max_q, causal, scale);
+  FwdArgs a;
+  a.out = (__nv_bfloat16*)out; a.lse = (float*)lse;
+  a.o_s = strides[6]; a.o_h = strides[7]; a.o_b = 0;
+  a.head_pair = fwd_head_pair(Hq, Hk);
+  const int per = a.head_pair ? BQ : 2 * BQ;
+  g.heads = a.head_pair ? Hq / 2 : Hq;
+  e = for_packed_launches(seqs, per, [](int nq, int) { return nq; },
+                          [&](int nq, int nk, int t) { return key_blocks(nq, nk, causal, t * per, per); },
+                          [&](const Packed& p, int n) { run_fwd(m, g, a, p, (long long)n * g.heads, sm_budget, stream); });
+  if (e != cudaSuccess) return (int)e;
+  e = cudaGetLastError();
+  if (e != cudaSuccess) set_last_error("dh_attn_fwd_packed launch failed: %s", cudaGetErrorString(e));
+  return (int)e;
 }
 
-// Scratch: delta [B*Hq*Sq] fp32 (row dot products of dO and O), rounded up to 256 bytes, then, when
-// the dK/dV kernel splits heads, the fp32 partials [2][hs][Sk][B][Hk][128].
 int64_t dh_attn_bwd_scratch_bytes(int B, int Hq, int Hk, int Sq, int Sk) {
-  int64_t n = ((int64_t)B * Hq * Sq * 4 + 255) / 256 * 256;
-  if (Hk > 0 && Hq % Hk == 0) {
-    const int hs = bwd_head_split(B, Hq, Hk, Sk);
-    if (hs > 1) n += (int64_t)2 * hs * Sk * B * Hk * D * 4;
-  }
-  return n;
+  const int hs = Hk > 0 && Hq % Hk == 0 ? bwd_head_split((long long)((Sk + BKV - 1) / BKV) * B, Hq, Hk) : 1;
+  return scratch_bytes(B, Hq, Hk, Sq, Sk, hs);
+}
+
+int64_t dh_attn_bwd_packed_scratch_bytes(int nseq, const int* cu_k, int Hq, int Hk, int Tq, int Tk) {
+  const int hs = Hk > 0 && Hq % Hk == 0 ? bwd_head_split(packed_kv_tiles(nseq, cu_k), Hq, Hk) : 1;
+  return scratch_bytes(1, Hq, Hk, Tq, Tk, hs);
 }
 
 int dh_attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* out, const void* lse, void* dq, void* dk,
                 void* dv, void* scratch, const int64_t* strides /* 8 tensors x (s,b,h): do,q,k,v,o,dq,dk,dv */, int B, int Hq, int Hk,
                 int Sq, int Sk, int d, int causal, float scale, int sm_budget, cudaStream_t stream) {
-  if (d != D) { set_last_error("dh_attn_bwd: head size %d is not supported (128 only)", d); return (int)cudaErrorInvalidValue; }
-  if (Hq % Hk != 0) { set_last_error("dh_attn_bwd: query heads must be a multiple of KV heads"); return (int)cudaErrorInvalidValue; }
+  if (!heads_ok("dh_attn_bwd", d, Hq, Hk)) return (int)cudaErrorInvalidValue;
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   const int64_t* sdo = strides; const int64_t* sq = strides + 3; const int64_t* sk = strides + 6; const int64_t* sv = strides + 9;
-  const int64_t* so = strides + 12; const int64_t* sdq = strides + 15; const int64_t* sdk = strides + 18; const int64_t* sdv = strides + 21;
-  const CUtensorMap* tq = tensor_map_sbhd(q, Sq, B, Hq, sq[0], sq[1], sq[2]);
-  const CUtensorMap* tk = tensor_map_sbhd(k, Sk, B, Hk, sk[0], sk[1], sk[2]);
-  const CUtensorMap* tv = tensor_map_sbhd(v, Sk, B, Hk, sv[0], sv[1], sv[2]);
-  const CUtensorMap* tdo = tensor_map_sbhd(dout, Sq, B, Hq, sdo[0], sdo[1], sdo[2]);
-  if (!tq || !tk || !tv || !tdo) return (int)cudaErrorInvalidValue;
-  static PerDeviceFlags configured_on;
-  bool& configured = device_flag(configured_on);
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
-    if (e != cudaSuccess) { set_last_error("dh_attn_bwd: shared memory opt-in failed: %s", cudaGetErrorString(e)); return (int)e; }
-    configured = true;
-  }
-  float* delta = reinterpret_cast<float*>(scratch);
+  const BwdMaps m = {tensor_map_sbhd(q, Sq, B, Hq, sq[0], sq[1], sq[2]), tensor_map_sbhd(k, Sk, B, Hk, sk[0], sk[1], sk[2]),
+                     tensor_map_sbhd(v, Sk, B, Hk, sv[0], sv[1], sv[2]), tensor_map_sbhd(dout, Sq, B, Hq, sdo[0], sdo[1], sdo[2])};
+  if (!m.q || !m.k || !m.v || !m.dout) return (int)cudaErrorInvalidValue;
+  cudaError_t e = opt_in_bwd<Dense>();
+  if (e != cudaSuccess) return (int)e;
   const long long rows_ll = (long long)B * Hq * Sq;
-  if (rows_ll > (1ll << 26)) {     // the delta grid (one warp per row) and the int row index stay well inside 32 bits
+  if (rows_ll > (1ll << 26)) {     // statistics are indexed well inside 32 bits
     set_last_error("dh_attn_bwd: B*Hq*Sq = %lld rows exceed the supported 2^26", rows_ll);
     return (int)cudaErrorInvalidValue;
   }
-  const int rows = (int)rows_ll;
-  attn_delta_kernel<<<(unsigned)((rows_ll * 32 + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, B, Hq, Sq,
-                                                                 sdo[0], sdo[1], sdo[2], so[0], so[1], so[2]);
-  DeviceStatus* st = reinterpret_cast<DeviceStatus*>(dh_status_device_ptr());
-  BwdGeometry g;
-  g.B = B; g.Hq = Hq; g.Hk = Hk; g.Sq = Sq; g.Sk = Sk; g.causal = causal; g.scale = scale;
-  g.dk_s = sdk[0]; g.dk_b = sdk[1]; g.dk_h = sdk[2]; g.dv_s = sdv[0]; g.dv_b = sdv[1]; g.dv_h = sdv[2];
-  g.status = st;
-  g.hs = bwd_head_split(B, Hq, Hk, Sk);
-  g.part = g.hs > 1 ? reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + ((int64_t)rows * 4 + 255) / 256 * 256) : nullptr;
-  g.x0 = 0; g.p0 = 0; g.ny = Hk * g.hs;
-  // DHELLAM_ATTN_BWD_T=1 (or dh_attn_set_bwd_mode(1)) selects the pipelined (transposed-score) form of the dK/dV kernel
-  if (g_bwd_mode < 0) {
-    const char* ev = getenv("DHELLAM_ATTN_BWD_T");
-    g_bwd_mode = ev ? atoi(ev) : 0;
+  const int hs = bwd_head_split((long long)((Sk + BKV - 1) / BKV) * B, Hq, Hk);
+  return bwd_common(dout, out, lse, dq, dk, dv, scratch, strides, m, geometry(B, Hq, Hk, Sq, Sk, Sq, Sk, Sq, causal, scale), hs, nullptr, sm_budget,
+                    stream);
+}
+
+int dh_attn_bwd_packed(const void* dout, const void* q, const void* k, const void* v, const void* out, const void* lse, void* dq, void* dk,
+                       void* dv, void* scratch, const int64_t* strides /* as dh_attn_bwd; the batch strides are not used */, int nseq,
+                       const int* cu_q, const int* cu_k, int Tq, int Tk, int lse_rows, int Hq, int Hk, int d, int causal, float scale,
+                       int sm_budget, cudaStream_t stream) {
+  if (!heads_ok("dh_attn_bwd_packed", d, Hq, Hk)) return (int)cudaErrorInvalidValue;
+  if (nseq <= 0 || Tq <= 0 || Tk <= 0) return 0;
+  const Sequences seqs = {nseq, cu_q, cu_k};
+  if (!offsets_ok("dh_attn_bwd_packed", seqs, Tq, Tk, lse_rows)) return (int)cudaErrorInvalidValue;
+  if ((long long)Hq * Tq > (1ll << 26)) {
+    set_last_error("dh_attn_bwd_packed: %lld query rows exceed the supported 2^26", (long long)Hq * Tq);
+    return (int)cudaErrorInvalidValue;
   }
-  if (g_bwd_mode == 1) {
-    const CUtensorMap* tq64 = tensor_map_sbhd(q, Sq, B, Hq, sq[0], sq[1], sq[2], BQT);
-    const CUtensorMap* tdo64 = tensor_map_sbhd(dout, Sq, B, Hq, sdo[0], sdo[1], sdo[2], BQT);
-    if (!tq64 || !tdo64) return (int)cudaErrorInvalidValue;
-    static PerDeviceFlags configured_t_on;
-    bool& configured_t = device_flag(configured_t_on);
-    if (!configured_t) {
-      cudaError_t e2 = cudaFuncSetAttribute(attn_bwd_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWDT_SMEM);
-      if (e2 != cudaSuccess) { set_last_error("dh_attn_bwd: shared memory opt-in failed: %s", cudaGetErrorString(e2)); return (int)e2; }
-      configured_t = true;
-    }
-    launch_in_waves((Sk + BKV - 1) / BKV, Hk * g.hs, B, sm_budget, [&](dim3 grid, int x0, int p0) {
-      g.x0 = x0; g.p0 = p0;
-      attn_bwd_t_kernel<<<grid, BWD_THREADS, BWDT_SMEM, stream>>>(*tq64, *tk, *tv, *tdo64, (const float*)lse, delta, (__nv_bfloat16*)dk,
-                                                                  (__nv_bfloat16*)dv, g);
-    });
-  } else {
-    launch_in_waves((Sk + BKV - 1) / BKV, Hk * g.hs, B, sm_budget, [&](dim3 grid, int x0, int p0) {
-      g.x0 = x0; g.p0 = p0;
-      attn_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, stream>>>(*tq, *tk, *tv, *tdo, (const float*)lse, delta, (__nv_bfloat16*)dk,
-                                                               (__nv_bfloat16*)dv, g);
-    });
-  }
-  if (g.hs > 1) {
-    const long long n = 2LL * Sk * B * Hk * (D / 8);
-    attn_dkv_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(g.part, g.hs, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, Sk, B, Hk,
-                                                                           sdk[0], sdk[1], sdk[2], sdv[0], sdv[1], sdv[2]);
-  }
-  DqGeometry gq;
-  gq.B = B; gq.Hq = Hq; gq.Hk = Hk; gq.Sq = Sq; gq.Sk = Sk; gq.causal = causal; gq.scale = scale;
-  gq.dq_s = sdq[0]; gq.dq_b = sdq[1]; gq.dq_h = sdq[2];
-  gq.status = st;
-  gq.ny = Hq;
-  launch_in_waves((Sq + BQ - 1) / BQ, Hq, B, sm_budget, [&](dim3 grid, int x0, int p0) {
-    gq.x0 = x0; gq.p0 = p0;
-    attn_bwd_dq_kernel<<<grid, BWD_THREADS, DQ_SMEM, stream>>>(*tq, *tk, *tv, *tdo, (const float*)lse, delta, (__nv_bfloat16*)dq, gq);
-  });
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) set_last_error("dh_attn_bwd launch failed: %s", cudaGetErrorString(e));
-  return (int)e;
+  const int64_t* sdo = strides; const int64_t* sq = strides + 3; const int64_t* sk = strides + 6; const int64_t* sv = strides + 9;
+  const BwdMaps m = {tensor_map_sbhd(q, Tq, 1, Hq, sq[0], sq[0], sq[2]), tensor_map_sbhd(k, Tk, 1, Hk, sk[0], sk[0], sk[2]),
+                     tensor_map_sbhd(v, Tk, 1, Hk, sv[0], sv[0], sv[2]), tensor_map_sbhd(dout, Tq, 1, Hq, sdo[0], sdo[0], sdo[2])};
+  if (!m.q || !m.k || !m.v || !m.dout) return (int)cudaErrorInvalidValue;
+  cudaError_t e = opt_in_bwd<Packed>();
+  if (e != cudaSuccess) return (int)e;
+  const int hs = bwd_head_split(packed_kv_tiles(nseq, cu_k), Hq, Hk);
+  return bwd_common(dout, out, lse, dq, dk, dv, scratch, strides, m, geometry(1, Hq, Hk, 0, 0, Tq, Tk, lse_rows, causal, scale), hs, &seqs,
+                    sm_budget, stream);
 }
 
 }  // extern "C"
@@ -1319,9 +1475,8 @@ extern "C" int dh_attn_bwd_noalloc(const void* dout, const void* q, const void* 
     void* ptr = nullptr;
     e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
     if (e != cudaSuccess || ptr == nullptr) { set_last_error("dh_attn_bwd_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e)); return (int)e; }
-    e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
-    if (e != cudaSuccess) { set_last_error("dh_attn_bwd_noalloc: shared memory opt-in failed: %s", cudaGetErrorString(e)); return (int)e; }
+    e = opt_in_bwd<Dense>();
+    if (e != cudaSuccess) return (int)e;
     g_noalloc_addr[dev] = ptr;
     g_noalloc_ready[dev] = true;
   }
@@ -1332,27 +1487,9 @@ extern "C" int dh_attn_bwd_noalloc(const void* dout, const void* q, const void* 
   if (!map_sbhd_into(&tq, q, Sq, B, Hq, sq) || !map_sbhd_into(&tk, k, Sk, B, Hk, sk) || !map_sbhd_into(&tv, v, Sk, B, Hk, sv) ||
       !map_sbhd_into(&tdo, dout, Sq, B, Hq, sdo))
     return (int)cudaErrorInvalidValue;
-  // delta is fully rewritten by every call, so nothing in the shared array needs clearing
-  float* delta = reinterpret_cast<float*>(g_noalloc_addr[dev]);
-  attn_delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, B,
-                                                                             Hq, Sq, sdo[0], sdo[1], sdo[2], so[0], so[1], so[2]);
-  BwdGeometry g;
-  g.B = B; g.Hq = Hq; g.Hk = Hk; g.Sq = Sq; g.Sk = Sk; g.causal = causal; g.scale = scale;
-  g.dk_s = sdk[0]; g.dk_b = sdk[1]; g.dk_h = sdk[2]; g.dv_s = sdv[0]; g.dv_b = sdv[1]; g.dv_h = sdv[2];
+  // delta is fully rewritten by every call, so nothing in the shared array needs clearing; the array holds delta only,
+  // so the query heads are never split here
+  Geometry g = geometry(B, Hq, Hk, Sq, Sk, Sq, Sk, Sq, causal, scale);
   g.status = nullptr;
-  g.hs = 1;              // the built-in scratch holds delta only: no head split here
-  g.part = nullptr;
-  g.x0 = 0; g.p0 = 0; g.ny = Hk;
-  attn_bwd_kernel<<<dim3((Sk + BKV - 1) / BKV, Hk, B), BWD_THREADS, BWD_SMEM, stream>>>(tq, tk, tv, tdo, (const float*)lse, delta,
-                                                                                      (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, g);
-  DqGeometry gq;
-  gq.B = B; gq.Hq = Hq; gq.Hk = Hk; gq.Sq = Sq; gq.Sk = Sk; gq.causal = causal; gq.scale = scale;
-  gq.dq_s = sdq[0]; gq.dq_b = sdq[1]; gq.dq_h = sdq[2];
-  gq.status = nullptr;
-  gq.x0 = 0; gq.p0 = 0; gq.ny = Hq;
-  attn_bwd_dq_kernel<<<dim3((Sq + BQ - 1) / BQ, Hq, B), BWD_THREADS, DQ_SMEM, stream>>>(tq, tk, tv, tdo, (const float*)lse, delta,
-                                                                                      (__nv_bfloat16*)dq, gq);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) set_last_error("dh_attn_bwd_noalloc launch failed: %s", cudaGetErrorString(e));
-  return (int)e;
+  return bwd_common(dout, out, lse, dq, dk, dv, g_noalloc_addr[dev], strides, BwdMaps{&tq, &tk, &tv, &tdo}, g, 1, nullptr, 0, stream);
 }

@@ -141,8 +141,7 @@ def merge_attention_partials(o_a, lse_a, o_b, lse_b):
 
 # ----------------------------------------------------------------------------- variable-length API
 def set_attn_bwd_mode(mode: int):
-    """dK/dV kernel on the GPU: 0 = one 128-query tile per iteration (default), 1 = the pipelined
-    transposed-score form, -1 = re-read ``DHELLAM_ATTN_BWD_T`` at the next call."""
+    """Accepted and without effect: the dK/dV kernel has one form."""
     K.proto("dh_attn_set_bwd_mode", [c_int], None)(int(mode))
 
 
@@ -165,18 +164,37 @@ def _as_sbhd(t, b, s):
     return t.view(b, s, t.shape[1], t.shape[2]).permute(1, 0, 2, 3)
 
 
+def _runs_packed(q, k, cq, ck, max_q) -> bool:
+    """Whether a packed batch runs as ONE launch of the packed kernels (offsets as kernel parameters, tiles of all
+    sequences in descending order of work): CUDA tensors with offsets that ascend and stay inside the tensors and
+    within ``max_q``.  Everything else (CPU, library backend, offsets that do not describe the tensors) takes the
+    sequence-by-sequence path, which also reports what is wrong with them."""
+    if not K.use_native(q) or len(cq) < 2 or len(cq) != len(ck) or q.dim() != 3 or k.dim() != 3:
+        return False
+    for c, rows in ((cq, q.shape[0]), (ck, k.shape[0])):
+        if c[0] < 0 or c[-1] > rows or any(c[i] > c[i + 1] for i in range(len(c) - 1)):
+            return False
+        n = _uniform_length(c)
+        if n and n * (len(c) - 1) != rows:
+            return False
+    return all(cq[i + 1] - cq[i] <= max_q for i in range(len(cq) - 1))
+
+
 def pymha_varlen_fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, p_dropout: float = 0.0,
                      softmax_scale: float | None = None, is_causal: bool = True, return_softmax: bool = False,
                      math_sm_count: int = 0, profiling: bool = False):
     """Packed variable-length attention with the reference's signature
     (csrc/operators/ops.h:18-32): ``q [total_q, h, d]``, ``k, v [total_k, h_k, d]`` and
     cumulative sequence offsets.  Returns ``(out [total_q, h, d], softmax_lse [b, h, max_q])``.
-    A batch of equal-length sequences runs as ONE launch over strided views of the packed tensors; sequences
-    of different lengths run one strided call each, so no padding copy is made.  Attention dropout is not supported by the sm_100a kernel (``p_dropout`` must be 0)."""
+    The whole batch is one launch, whatever the lengths.  Attention dropout is not supported by the sm_100a kernel
+    (``p_dropout`` must be 0)."""
     assert p_dropout == 0.0, "attention dropout is not implemented"
     cq = _offsets(cu_seqlens_q)
     ck = _offsets(cu_seqlens_k)
     b = len(cq) - 1
+    if _runs_packed(q, k, cq, ck, max_seqlen_q):
+        from .attention_native import attn_fwd_packed
+        return attn_fwd_packed(q, k, v, cq, ck, max_seqlen_q, is_causal, softmax_scale, abs(math_sm_count))
     sq, sk = _uniform_length(cq), _uniform_length(ck)
     if sq and sk and sq == max_seqlen_q:
         # every sequence has the same length (the reference's own use: a micro-batch of fixed-length samples):
@@ -202,6 +220,10 @@ def pymha_varlen_bwd(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k
     ck = _offsets(cu_seqlens_k)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     b = len(cq) - 1
+    if softmax_lse.dim() == 3 and softmax_lse.shape[:2] == (b, q.shape[1]) and _runs_packed(q, k, cq, ck, softmax_lse.shape[2]):
+        from .attention_native import attn_bwd_packed
+        attn_bwd_packed(dout, q, k, v, out, softmax_lse, dq, dk, dv, cq, ck, is_causal, softmax_scale, abs(math_sm_count))
+        return dq, dk, dv
     sq, sk = _uniform_length(cq), _uniform_length(ck)
     if sq and sk and sq == max_seqlen_q and softmax_lse.shape[-1] == sq:
         a, b_, c = attn_bwd(_as_sbhd(dout, b, sq), _as_sbhd(q, b, sq), _as_sbhd(k, b, sk), _as_sbhd(v, b, sk), _as_sbhd(out, b, sq),

@@ -9,6 +9,7 @@ does not allocate.
 from __future__ import annotations
 
 import ctypes
+import math
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
@@ -43,3 +44,52 @@ def attn_bwd_native(dout, q, k, v, out, lse, dq, dk, dv, causal, scale, sm_budge
     K.check(fn(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), dq.data_ptr(),
                dk.data_ptr(), dv.data_ptr(), scratch.data_ptr(), arr, B, Hq, Hk, Sq, Sk, d, 1 if causal else 0, scale,
                sm_budget, K.stream_ptr(stream)), "dh_attn_bwd")
+
+
+def _packed_offsets(cu):
+    return (c_int * len(cu))(*cu)
+
+
+def attn_fwd_packed(q, k, v, cq, ck, max_q, causal, scale, sm_budget=0, stream=None):
+    """Packed batch in one launch: ``q [Tq, Hq, d]``, ``k, v [Tk, Hk, d]``, offsets as Python lists (checked by the
+    caller).  Returns ``(out like q, lse [b, Hq, max_q])``; statistics past a sequence's end are ``-inf``."""
+    Tq, Hq, d = q.shape
+    Tk, Hk = k.shape[0], k.shape[1]
+    assert q.stride(2) == 1 and k.stride(2) == 1 and v.stride(2) == 1
+    scale = scale if scale is not None else 1.0 / math.sqrt(d)
+    out = torch.empty_like(q)
+    assert out.stride(2) == 1
+    b = len(cq) - 1
+    whole = all(cq[i + 1] - cq[i] == max_q for i in range(b))
+    shape = (b, Hq, max_q)
+    lse = torch.empty(shape, dtype=torch.float32, device=q.device) if whole else \
+        torch.full(shape, float("-inf"), dtype=torch.float32, device=q.device)
+    strides = (c_int64 * 8)(*(s for t in (q, k, v, out) for s in (t.stride(0), t.stride(1))))
+    fn = K.proto("dh_attn_fwd_packed", [c_void_p] * 5 + [ctypes.POINTER(c_int64), c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int),
+                                                         c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
+    K.check(fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), strides, b, _packed_offsets(cq),
+               _packed_offsets(ck), Tq, Tk, max_q, Hq, Hk, d, 1 if causal else 0, scale, sm_budget, K.stream_ptr(stream)),
+            "dh_attn_fwd_packed")
+    return out, lse
+
+
+def attn_bwd_packed(dout, q, k, v, out, lse, dq, dk, dv, cq, ck, causal, scale, sm_budget=0, stream=None):
+    """Backward of ``attn_fwd_packed`` into ``dq, dk, dv``."""
+    Tq, Hq, d = q.shape
+    Tk, Hk = k.shape[0], k.shape[1]
+    strides = []
+    for t in (dout, q, k, v, out, dq, dk, dv):
+        assert t.stride(2) == 1 and t.dtype == torch.bfloat16
+        strides += [t.stride(0), t.stride(0), t.stride(1)]
+    scale = scale if scale is not None else 1.0 / math.sqrt(d)
+    lse = lse.contiguous()
+    b = len(cq) - 1
+    cu_q, cu_k = _packed_offsets(cq), _packed_offsets(ck)
+    p_int = ctypes.POINTER(c_int)
+    nbytes = K.proto("dh_attn_bwd_packed_scratch_bytes", [c_int, p_int, c_int, c_int, c_int, c_int], c_int64)
+    scratch = _scratch_for(q.device, nbytes(b, cu_k, Hq, Hk, Tq, Tk))
+    fn = K.proto("dh_attn_bwd_packed", [c_void_p] * 10 + [ctypes.POINTER(c_int64), c_int, p_int, p_int, c_int, c_int, c_int, c_int, c_int,
+                                                          c_int, c_int, c_float, c_int, c_void_p])
+    K.check(fn(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), dq.data_ptr(),
+               dk.data_ptr(), dv.data_ptr(), scratch.data_ptr(), (c_int64 * 24)(*strides), b, cu_q, cu_k, Tq, Tk, lse.shape[2], Hq,
+               Hk, d, 1 if causal else 0, scale, sm_budget, K.stream_ptr(stream)), "dh_attn_bwd_packed")

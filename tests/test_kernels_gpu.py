@@ -327,6 +327,40 @@ def test_varlen_api_with_equal_lengths_uses_strided_views_of_the_packed_tensors(
         assert rel(sb(a), r) < 1e-3
 
 
+@pytest.mark.parametrize("hq,hk", [(4, 2), (3, 1), (2, 2)])
+@pytest.mark.parametrize("ql,kl,causal", [([1, 127, 128, 129, 300], None, True), ([130, 64, 257], [130, 200, 513], True),
+                                          ([65, 0, 256], [40, 7, 300], False), ([17] * 150, None, True)])
+def test_packed_attention_against_fp32_sequence_by_sequence(ql, kl, causal, hq, hk):
+    """Ragged batches in one launch (and, with 150 sequences, in two): tiles that end inside a sequence, an empty
+    sequence, more keys than queries, odd and even groups; the tolerances are those of the dense test above (bf16
+    probabilities and outputs).  One sequence holds NaN: nothing of it may reach its neighbours."""
+    from dhellam_b200.ops.attention import attn_bwd, attn_fwd, pymha_varlen_bwd, pymha_varlen_fwd
+    kl, d = kl or ql, 128
+    off = lambda n: [sum(n[:i]) for i in range(len(n) + 1)]
+    cq, ck = off(ql), off(kl)
+    q, k, v, do = bf(cq[-1], hq, d), bf(ck[-1], hk, d), bf(ck[-1], hk, d), bf(cq[-1], hq, d)
+    sick = 2                                               # between two healthy ones (or the last)
+    for t, c in ((q, cq), (k, ck), (v, ck), (do, cq)):
+        t[c[sick]:c[sick + 1]] = float("nan")
+    out, lse = pymha_varlen_fwd(q, k, v, cq, ck, max(ql), max(kl), is_causal=causal)
+    dq, dk, dv = pymha_varlen_bwd(do, q, k, v, out, lse, cq, ck, max(ql), max(kl), is_causal=causal)
+    assert lse.shape == (len(ql), hq, max(ql))
+    cpu = lambda t, c, i: t[c[i]:c[i + 1]].unsqueeze(1).float().cpu()
+    got, want = [[] for _ in range(5)], [[] for _ in range(5)]
+    for i in range(len(ql)):
+        if i == sick or ql[i] == 0:
+            continue
+        qi, ki, vi, di = cpu(q, cq, i), cpu(k, ck, i), cpu(v, ck, i), cpu(do, cq, i)
+        o, l = attn_fwd(qi, ki, vi, causal)
+        grads = attn_bwd(di, qi, ki, vi, o, l, causal)
+        mine = (cpu(out, cq, i), lse[i:i + 1, :, :ql[i]].cpu(), cpu(dq, cq, i), cpu(dk, ck, i), cpu(dv, ck, i))
+        for a, b, x, y in zip(got, want, mine, (o, l) + tuple(grads)):
+            a.append(x.flatten())
+            b.append(y.flatten())
+    for name, a, b, tol in zip(("out", "lse", "dq", "dk", "dv"), got, want, (1e-2, 1e-3, 2e-2, 2e-2, 2e-2)):
+        assert rel(torch.cat(a), torch.cat(b)) < tol, (name, rel(torch.cat(a), torch.cat(b)))
+
+
 def test_bounded_wait_reports_timeout_without_hanging():
     """A flag that nobody sets: the device-side wait gives up after its (short) budget and
     the host reads the status word; the context stays usable."""
