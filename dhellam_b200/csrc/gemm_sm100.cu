@@ -491,7 +491,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint8_t* sEpi = smem + p.stages * STAGE2_BYTES;
   Control2* ctl = reinterpret_cast<Control2*>(smem + p.stages * STAGE2_BYTES + EPI_BYTES);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();          // 0 = leader
   const int pair_id = blockIdx.x >> 1;
@@ -522,7 +522,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   __syncthreads();
   cluster_sync_all();
   tc_fence_after();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort_flag;
   if (p.start_id != 0 && threadIdx.x == 0) {
     if (atomicAdd(&g_start_count, 1u) + 1u == gridDim.x) {       // the last CTA to become resident
@@ -583,8 +583,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) --------------
-    if (lane == 0 && rank == 0) {
+    // The whole warp walks the loop and one elected lane issues under a predicate, so that descriptors and barrier
+    // addresses live in uniform registers.  Issued inside a divergent branch the four products and two commits of a
+    // k-block took about as long to issue as the 512 cycles they execute.
+    if (rank == 0) {
       constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t leader = elect_one();
       int s = 0;
       uint32_t ph = 0;
       int acc = 0;
@@ -594,11 +598,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const Item im = item_coords(it, p, num_tiles, num_kb);
         const int kb0 = im.kb0, kb1 = im.kb1;
         if (kb0 >= kb1) continue;                       // an expert without rows: nothing to add (all roles skip the item)
-        if (!mbar_wait<true>(&ctl->acc_empty[acc], acc_ph ^ 1, abort_flag, p.status, 210, p.wait_budget)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait<true>(&ctl->acc_empty[acc], acc_ph ^ 1, abort_flag, p.status, 210, p.wait_budget))) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * ACC_COLS;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&ctl->full[s], ph, abort_flag, p.status, 211, p.wait_budget)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(&ctl->full[s], ph, abort_flag, p.status, 211, p.wait_budget))) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_base = smem_u32(sA + s * A2_STAGE_BYTES);
           const uint32_t b_base = smem_u32(sB + s * B2_STAGE_BYTES);
@@ -608,17 +612,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                                         : umma_smem_desc(a_base + kk * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? umma_smem_desc(b_base + kk * 2048, BK * 128, 1024)
                                         : umma_smem_desc(b_base + kk * 32, 16, 1024);
-            umma_bf16_2sm(tmem_acc, adesc, bdesc, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
+            umma_bf16_2sm_by(leader, tmem_acc, adesc, bdesc, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
           }
           const uint32_t e = smem_u32(&ctl->empty[s]);
-          umma_commit_2sm(mapa_u32(e, 0));
-          umma_commit_2sm(mapa_u32(e, 1));
+          umma_commit_2sm_by(leader, mapa_u32(e, 0));
+          umma_commit_2sm_by(leader, mapa_u32(e, 1));
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
         const uint32_t f = smem_u32(&ctl->acc_full[acc]);
-        umma_commit_2sm(mapa_u32(f, 0));
-        umma_commit_2sm(mapa_u32(f, 1));
+        umma_commit_2sm_by(leader, mapa_u32(f, 0));
+        umma_commit_2sm_by(leader, mapa_u32(f, 1));
         if (++acc == NUM_ACC) { acc = 0; acc_ph ^= 1; }
       }
     }
