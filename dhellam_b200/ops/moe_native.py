@@ -93,7 +93,7 @@ class DeviceMoE:
         self.calls = {s: 0 for s in SITES}
         self.total = {s: [0, 0] for s in SITES}
         self._arr = ctypes.c_void_p * self.ep
-        self.ctas = int(os.environ.get("DHELLAM_MOE_CTAS", "64"))
+        self.ctas = int(os.environ.get("DHELLAM_MOE_CTAS", "0"))      # 0 = by the number of ranks (csrc/moe_sm100.cu)
 
     # ------------------------------------------------------------------ helpers
     def _ptr_array(self, off):
