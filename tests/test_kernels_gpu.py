@@ -234,6 +234,29 @@ def attn_bwd_mode(request):
     set_attn_bwd_mode(0)
 
 
+@pytest.mark.parametrize("rows,h", [(1, 8), (3, 264), (700, 1000), (5, 8192), (4, 8200), (2, 16384)])
+@pytest.mark.parametrize("kind", ["rms", "layer"])
+def test_norm_backward_row_lengths(rows, h, kind):
+    """One vector per thread (up to 8192 elements, lanes to spare at 264 and 1000), several beyond; more rows than CTAs; with and
+    without a residual, and a gradient buffer that is only 4-byte aligned.  bf16 results: 1e-2; fp32 sums: 1e-3."""
+    from dhellam_b200.ops.norm import layernorm_bwd, layernorm_fwd, rmsnorm_bwd, rmsnorm_fwd
+    x, w, b, dy, res = bf(rows, h), bf(h), bf(h), bf(rows, h), bf(rows, h)
+    grads = torch.zeros(2, h + 1, device=DEV)
+    dw, db, dwr, dbr = grads[0, 1:], grads[1, 1:], torch.zeros(h), torch.zeros(h)
+    cpu = lambda *t: [a.cpu().float() for a in t]
+    xc, wc, bc, dyc, rc = cpu(x, w, b, dy, res)
+    if kind == "rms":
+        _, rstd = rmsnorm_fwd(x, w)
+        dx, _ = rmsnorm_bwd(dy, x, w, rstd, weight_main_grad=dw, residual_grad=res)
+        dxr, _ = rmsnorm_bwd(dyc, xc, wc, rstd.cpu(), weight_main_grad=dwr, residual_grad=rc)
+    else:
+        _, mu, rstd = layernorm_fwd(x, w, b)
+        dx, _, _ = layernorm_bwd(dy, x, w, mu, rstd, weight_main_grad=dw, bias_main_grad=db)
+        dxr, _, _ = layernorm_bwd(dyc, xc, wc, mu.cpu(), rstd.cpu(), weight_main_grad=dwr, bias_main_grad=dbr)
+        assert rel(db, dbr) < 1e-3
+    assert rel(dx, dxr) < 1e-2 and rel(dw, dwr) < 1e-3
+
+
 @pytest.mark.parametrize("Sq,Sk,B,Hq,Hk,causal", [(128, 128, 1, 1, 1, True), (256, 256, 2, 4, 2, True), (384, 384, 1, 2, 1, False),
                                                      (200, 200, 2, 2, 2, True), (128, 256, 1, 2, 1, False), (256, 128, 1, 2, 2, False)])
 def test_attention_forward_backward(Sq, Sk, B, Hq, Hk, causal, attn_bwd_mode):
