@@ -20,7 +20,7 @@ _scratch = {}
 
 
 def _scratch_for(device, nbytes: int):
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, K.current_raw_stream(device))
     buf = _scratch.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(nbytes, dtype=torch.uint8, device=device)

@@ -158,6 +158,8 @@ def gemm_tn_acc(dy, x, main_grad, accumulate: bool = True, sm_budget: int = 0, s
 def _timed(fn, profiling, stream):
     """Runs ``fn`` on ``stream``; returns ``(result, elapsed ms or 0)`` timed with CUDA events
     on that stream (the reference wraps its calls in host timers, layernorm_column.py:28-35)."""
+    if not profiling and stream is None:       # the current stream, nothing to time
+        return fn(), 0.0
     if not torch.cuda.is_available():
         return fn(), 0.0
     stream = stream if stream is not None else torch.cuda.current_stream()

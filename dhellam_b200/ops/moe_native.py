@@ -113,16 +113,16 @@ class DeviceMoE:
         return self.ptrs[self.rank] + self.off_cnt[site][slot]
 
     def _wait(self, site, slot):
-        s = torch.cuda.current_stream(self.device)
+        s = K.current_raw_stream(self.device)
         fn = K.proto("dh_wait_counters", [c_void_p, c_int, c_uint, c_int64, c_void_p])
-        K.check(fn(self._counter_ptr(site, slot), 1, self.total[site][slot], 0, s.cuda_stream), "dh_wait_counters")
+        K.check(fn(self._counter_ptr(site, slot), 1, self.total[site][slot], 0, s), "dh_wait_counters")
 
     # ------------------------------------------------------------------ plan
     def plan(self, topi32) -> DevicePlan:
         n = topi32.numel()
         T = n // self.k
         dev = self.device
-        s = torch.cuda.current_stream(dev).cuda_stream
+        s = K.current_raw_stream(dev)
         pos = torch.empty(n, dtype=torch.int32, device=dev)
         counts = torch.empty(self.E, dtype=torch.int32, device=dev)
         K.check(K.proto("dh_moe_plan", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])(
@@ -147,7 +147,7 @@ class DeviceMoE:
         """Pushes ``src_rows[i // k]`` (optionally scaled per copy) of every copy to its owner's landing
         buffer of ``site``.  Returns ``(slot, dots)``; ``dots [T*k]`` = row-wise dot with ``other`` if given."""
         slot = self.next_slot(site)
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = K.current_raw_stream(self.device)
         K.check(K.proto("dh_moe_zero_pad", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])(
             self.view(site, slot).data_ptr(), plan.offs.data_ptr(), plan.rows_e.data_ptr(), self.el, self.h, s), "dh_moe_zero_pad")
         n = plan.topi.numel()
@@ -174,14 +174,14 @@ class DeviceMoE:
 
     def publish(self, site: str, slot: int):
         """After the kernel that filled the output buffer on the current stream: tells every rank it is complete."""
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = K.current_raw_stream(self.device)
         self.total[site][slot] += self.ep
         K.check(K.proto("dh_announce", [c_void_p, c_int, c_uint, c_void_p])(self._ptr_array(self.off_cnt[site][slot]), self.ep, 1, s),
                 "dh_announce")
 
     def combine(self, plan: DevicePlan, site: str, slot: int, gates=None, keep_copies: bool = False):
         """``out[t] = sum_j gates[t, j] * owner_buffer[copy (t, j)]`` (plain sum without gates)."""
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = K.current_raw_stream(self.device)
         out = torch.empty((plan.T, self.h), dtype=torch.bfloat16, device=self.device)
         copies = torch.empty((plan.T * self.k, self.h), dtype=torch.bfloat16, device=self.device) if keep_copies else None
         fn = K.proto("dh_moe_combine", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_uint, c_int, c_int, c_int,
@@ -193,7 +193,7 @@ class DeviceMoE:
 
     # ------------------------------------------------------------------ grouped GEMMs
     def _grouped(self, a, b2d, b_mn, d, M, N, Kd, mode, plan, budget):
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = K.current_raw_stream(self.device)
         fn = K.proto("dh_gemm_grouped_bf16", [c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int, c_int, c_int, c_int,
                                               c_int, c_void_p, c_int, c_int, c_void_p])
         K.check(fn(a.data_ptr(), a.stride(0), b2d.data_ptr(), b2d.stride(0), int(b_mn), d.data_ptr(), d.stride(0), M, N, Kd, self.el, mode,
@@ -226,7 +226,7 @@ class DeviceMoE:
     def swiglu_fwd(self, z, plan):
         f = z.shape[1] // 2
         out = torch.empty((self.capacity, f), dtype=z.dtype, device=z.device)
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = K.current_raw_stream(self.device)
         K.check(K.proto("dh_swiglu_fwd_n", [c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int, c_void_p])(
             z.data_ptr(), out.data_ptr(), self.capacity, plan.offs[self.el:].data_ptr(), f, 0, s), "dh_swiglu_fwd_n")
         return out
@@ -234,7 +234,7 @@ class DeviceMoE:
     def swiglu_bwd(self, d_a, z, plan):
         f = z.shape[1] // 2
         dz = torch.empty_like(z)
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = K.current_raw_stream(self.device)
         K.check(K.proto("dh_swiglu_bwd_n", [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int, c_void_p])(
             d_a.data_ptr(), z.data_ptr(), dz.data_ptr(), self.capacity, plan.offs[self.el:].data_ptr(), f, 0, s), "dh_swiglu_bwd_n")
         return dz

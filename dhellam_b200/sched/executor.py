@@ -19,6 +19,7 @@ from typing import Dict, List, Optional
 import torch
 
 from .ir import BWD, COMM, FWD, LayerProgram, LayerRun
+from .. import kernels as K
 from .strategy import CARRIED, CARRY_SUFFIX, Block, Strategy, split_budget
 
 
@@ -48,6 +49,27 @@ class StreamSet:
 
     def ctx(self, stream):
         return torch.cuda.stream(stream) if (self.cuda and stream is not None) else contextlib.nullcontext()
+
+    @contextlib.contextmanager
+    def restoring(self):
+        """Around ``switch_to``: the caller's current stream is current again afterwards."""
+        if not self.cuda:
+            yield
+            return
+        before = torch.cuda.current_stream()
+        try:
+            yield
+        finally:
+            torch.cuda.set_stream(before)
+
+    def switch_to(self, stream) -> bool:
+        """Makes ``stream`` current and leaves it so; False if that takes another device (then ``ctx`` has to be used).
+        A run of ops that share a stream thus pays for one switch instead of one save and restore per op."""
+        if not self.cuda or torch._C._cuda_getDevice() != stream.device_index:
+            return False
+        if K.current_raw_stream() != stream.cuda_stream:
+            torch.cuda.set_stream(stream)
+        return True
 
     def join_all_into(self, target):
         """Makes ``target`` wait for everything enqueued so far on the three streams."""
@@ -122,6 +144,7 @@ class Executor:
         self._lane_of: Dict[str, Dict[str, str]] = {}
         self._markers = program.marker_targets()
         self._carry_names = {f"{n}{CARRY_SUFFIX}": n for n in self._markers.values()}
+        self._switching = False                  # inside run(): the current stream follows the ops, run() restores it
         self._carry: List[tuple] = []            # weight-gradient ops handed to the next layer run
         for key, blocks in (("pair", self.strategy.dcblocks), ("fwd", self.strategy.fwd_only), ("bwd", self.strategy.bwd_only)):
             lanes = {}
@@ -173,19 +196,24 @@ class Executor:
                 return
             self._exec(op, run, lane, lanes, budget)
 
-        for blk in blocks:
-            for e in blk.s3:
-                launch(e, "S3")
-            fwd_comm = any(self.program.has(split_budget(e)[0]) and self.program.op(split_budget(e)[0]).strand == FWD
-                           for e in blk.s3)
-            order = (("S2", blk.s2), ("S1", blk.s1)) if fwd_comm else (("S1", blk.s1), ("S2", blk.s2))
-            for lane, lst in order:
-                for e in lst:
-                    launch(e, lane)
-            if self.sync_per_block:
-                torch.cuda.synchronize()
-        for target, (op, run, b) in list(pending.items()):   # flush what no marker claimed
-            self._exec(op, run, "S2", lanes, b)
+        with self.streams.restoring():
+            self._switching = True
+            try:
+                for blk in blocks:
+                    for e in blk.s3:
+                        launch(e, "S3")
+                    fwd_comm = any(self.program.has(split_budget(e)[0]) and self.program.op(split_budget(e)[0]).strand == FWD
+                                   for e in blk.s3)
+                    order = (("S2", blk.s2), ("S1", blk.s1)) if fwd_comm else (("S1", blk.s1), ("S2", blk.s2))
+                    for lane, lst in order:
+                        for e in lst:
+                            launch(e, lane)
+                    if self.sync_per_block:
+                        torch.cuda.synchronize()
+                for target, (op, run, b) in list(pending.items()):   # flush what no marker claimed
+                    self._exec(op, run, "S2", lanes, b)
+            finally:
+                self._switching = False
 
     def flush_carry(self, lane: Optional[str] = None):
         """Runs the ops that earlier layer runs handed over (on ``lane``, else on the lane they
@@ -239,7 +267,7 @@ class Executor:
             self._pre_events[op.name] = pre
         if self.nvtx:
             torch.cuda.nvtx.range_push(f"{'F' if op.strand == FWD else 'B'}:{op.name} L{run.layer_index} mb{getattr(run.mb, 'index', -1)}")
-        with st.ctx(stream):
+        with contextlib.nullcontext() if self._switching and st.switch_to(stream) else st.ctx(stream):
             if self.profile and st.cuda:
                 e0 = torch.cuda.Event(enable_timing=True)
                 e1 = torch.cuda.Event(enable_timing=True)
