@@ -817,6 +817,212 @@ static int launch_pair(const CUtensorMap* ta, const CUtensorMap* tb, const CUten
 }
 }  // namespace pair
 
+// ---------------------------------------------------------------------------------------
+// Small-output variant: 128 x 128 tiles, one CTA each, K divided over a cluster.
+//
+// A product of a few hundred tokens has few output tiles: 300 x 6144 is 48 tiles of 256 x 256 for 74 CTA pairs, each
+// walking the whole of K alone (29 us, where reading the weight takes 8).  Here the tile is a quarter of that and the
+// S <= 8 CTAs of a cluster each take 1 / S of K, so that the weight streams through all SMs at once.  Each CTA leaves
+// its fp32 partial tile in its own shared memory (the ring is done with), and after a cluster barrier CTA r adds rows
+// [128 r / S, 128 (r + 1) / S) of all S partials in a fixed order (distributed shared memory) and writes them: no workspace, no
+// atomics, the same result in every run.  Bounded by the stream of the larger operand; where many tiles fill the
+// machine the pair kernel reads half as much per product and wins (choose_cluster_k).
+// ---------------------------------------------------------------------------------------
+namespace small {
+constexpr int TILE_N = 128;
+constexpr int MAX_STAGES = 6;
+constexpr int A_BYTES = BM * BK * 2, B_BYTES = TILE_N * BK * 2;      // 16 KiB each
+constexpr int SLOT_BYTES = A_BYTES + B_BYTES;
+constexpr int ACC_LD = TILE_N + 4;                                   // fp32 partial tile: padded rows, conflict-free 16-byte stores
+constexpr int MIN_STAGES = (BM * ACC_LD * 4 + SLOT_BYTES - 1) / SLOT_BYTES;   // the partial tile reuses the ring
+constexpr int MAX_CLUSTER = 8;
+
+struct __align__(8) Control3 {
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
+  uint64_t done;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+constexpr int smem_bytes(int stages) { return stages * SLOT_BYTES + 1024 + 256; }
+
+struct SmallParams {
+  void* d;
+  int64_t ldd;
+  int M, N, K;
+  int tiles_m, cluster, stages, accumulate;
+  DeviceStatus* status;
+};
+
+template <bool A_MN, bool B_MN, bool OUT_F32>
+__global__ void __launch_bounds__(THREADS)
+gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const SmallParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Control3* ctl = reinterpret_cast<Control3*>(smem + p.stages * SLOT_BYTES);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / p.cluster, rank = blockIdx.x - tile * p.cluster;      // clusters are runs of consecutive CTAs
+  const int m0 = tile % p.tiles_m * BM, n0 = tile / p.tiles_m * TILE_N;               // tiles that share the weight are neighbours
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int kb0 = (int)((long long)rank * num_kb / p.cluster), kb1 = (int)((long long)(rank + 1) * num_kb / p.cluster);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
+    mbar_init(&ctl->done, 1);
+    ctl->abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) { tmem_alloc(&ctl->tmem_base, TILE_N); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
+  volatile int* abort_flag = &ctl->abort_flag;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_a);
+      tma_prefetch_desc(&tmap_b);
+      int s = 0;
+      uint32_t ph = 1;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&ctl->empty[s], ph, abort_flag, p.status, 120)) break;
+        mbar_expect_tx(&ctl->full[s], SLOT_BYTES);
+        uint8_t* a_dst = smem + s * SLOT_BYTES;
+        uint8_t* b_dst = a_dst + A_BYTES;
+        const int k0 = kb * BK;
+        if (A_MN) {
+#pragma unroll
+          for (int j = 0; j < BM / 64; ++j) tma_load_2d(a_dst + j * (BK * 128), &tmap_a, &ctl->full[s], m0 + 64 * j, k0);
+        } else {
+          tma_load_2d(a_dst, &tmap_a, &ctl->full[s], k0, m0);
+        }
+        if (B_MN) {
+#pragma unroll
+          for (int j = 0; j < TILE_N / 64; ++j) tma_load_2d(b_dst + j * (BK * 128), &tmap_b, &ctl->full[s], n0 + 64 * j, k0);
+        } else {
+          tma_load_2d(b_dst, &tmap_b, &ctl->full[s], k0, n0);
+        }
+        if (++s == p.stages) { s = 0; ph ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = umma_idesc_bf16(BM, TILE_N, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    const uint32_t leader = elect_one();
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&ctl->full[s], ph, abort_flag, p.status, 220))) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t a_base = smem_u32(smem + s * SLOT_BYTES), b_base = a_base + A_BYTES;
+#pragma unroll
+      for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+        const uint64_t adesc = A_MN ? umma_smem_desc(a_base + kk * 2048, BK * 128, 1024) : umma_smem_desc(a_base + kk * 32, 16, 1024);
+        const uint64_t bdesc = B_MN ? umma_smem_desc(b_base + kk * 2048, BK * 128, 1024) : umma_smem_desc(b_base + kk * 32, 16, 1024);
+        umma_bf16_by(leader, tmem_base, adesc, bdesc, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
+      }
+      umma_commit_by(leader, &ctl->empty[s]);
+      if (++s == p.stages) { s = 0; ph ^= 1; }
+    }
+    if (ok) umma_commit_by(leader, &ctl->done);
+  } else {
+    // partial tile -> this CTA's shared memory (all loads have landed and all products have read them)
+    const int quarter = warp & 3;
+    if (mbar_wait(&ctl->done, 0, abort_flag, p.status, 320)) {
+      tc_fence_after();
+      float* row = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * ACC_LD;
+#pragma unroll 1
+      for (int c = 0; c < TILE_N / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + c * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(row + c * 32 + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  cluster_sync_all();                      // all partial tiles of the cluster are in place
+  {
+    // row i of this CTA's share: a warp per row, four columns per lane
+    const int rows = BM / p.cluster;
+    const int col = n0 + 4 * lane;
+    for (int i = warp; i < rows; i += THREADS / 32) {
+      const int r = rank * rows + i;
+      if (m0 + r >= p.M) break;
+      const uint32_t local = smem_u32(smem) + (uint32_t)(r * ACC_LD + 4 * lane) * 4;
+      float4 part[MAX_CLUSTER];
+#pragma unroll
+      for (int k = 0; k < MAX_CLUSTER; ++k)
+        if (k < p.cluster) part[k] = ld_cluster_v4(mapa_u32(local, (uint32_t)k));
+      float4 v = part[0];
+#pragma unroll
+      for (int k = 1; k < MAX_CLUSTER; ++k)
+        if (k < p.cluster) { v.x += part[k].x; v.y += part[k].y; v.z += part[k].z; v.w += part[k].w; }
+      const float e[4] = {v.x, v.y, v.z, v.w};
+      if (OUT_F32) {
+        float* dst = reinterpret_cast<float*>(p.d) + (int64_t)(m0 + r) * p.ldd + col;
+        if (col + 4 <= p.N) {
+          if (p.accumulate) {
+            const float4 o = *reinterpret_cast<const float4*>(dst);
+            v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+          }
+          *reinterpret_cast<float4*>(dst) = v;
+        } else {
+          for (int j = 0; j < 4; ++j)
+            if (col + j < p.N) dst[j] = p.accumulate ? dst[j] + e[j] : e[j];
+        }
+      } else {
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.d) + (int64_t)(m0 + r) * p.ldd + col;
+        if (col + 4 <= p.N) {
+          *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+        } else {
+          for (int j = 0; j < 4; ++j)
+            if (col + j < p.N) dst[j] = __float2bfloat16(e[j]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();                      // no CTA leaves while another reads its shared memory
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, TILE_N); }
+}
+
+template <bool A_MN, bool B_MN, bool OUT_F32>
+static int launch_small(const CUtensorMap* ta, const CUtensorMap* tb, const SmallParams& p, int tiles, cudaStream_t stream) {
+  auto kern = gemm_small_kernel<A_MN, B_MN, OUT_F32>;
+  static PerDeviceFlags configured_on;
+  bool& configured = device_flag(configured_on);
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MAX_STAGES));
+    if (e != cudaSuccess) {
+      set_last_error("cudaFuncSetAttribute(smem=%d) failed: %s", smem_bytes(MAX_STAGES), cudaGetErrorString(e));
+      return (int)e;
+    }
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.cluster);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem_bytes(p.stages);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *ta, *tb, p);
+  if (e != cudaSuccess) set_last_error("small gemm launch failed: %s", cudaGetErrorString(e));
+  return (int)e;
+}
+}  // namespace small
+
 // 0 = choose per problem, 1 = single-CTA kernel only, 2 = CTA-pair kernel whenever M > 128.
 static int g_gemm_mode = -1;
 static int gemm_mode() {
@@ -870,6 +1076,30 @@ static int choose_split_k(int tiles, int pairs, int num_kb) {
   return best < 1 ? 1 : best;
 }
 
+// CTAs that share the K of one 128 x 128 tile, or 0 = the pair (or single-CTA) kernel is the faster one.
+// Forced by dh_gemm_set_cluster_k: -1 = this rule, 0 = never, n = n CTAs (as far as K allows).
+static int g_cluster_k = -1;
+
+// The rule, from a sweep of 8 to 2048 rows against weights of 512 x 512 to 28672 x 4096 (times with 10 us of launch and event
+// in them, pair kernel -> this one): up to a quarter of the SMs' worth of tiles, 4 CTAs per tile (128 x 4096 x 4096 36 -> 19 us,
+// 512 x 1024 x 1024 15.4 -> 12.3 us); up to half, 2, or 4 where K is long (200 x 4096 x 14336 78 -> 47 us, x 4096 31 -> 23 us); up to one
+// tile per SM, 2 where K is long enough to pay for the reduction (300 x 4096 x 14336 80 -> 66 us, 300 x 6144 x 4096 34 -> 32 us; but
+// 2048 x 1024 x 1024 15 -> 18 us). With more tiles the pair kernel's larger tiles read less through L2 and win (512 x 6144 x 4096 35
+// against 45 us), as it does for fp32 outputs of more than one row of tiles (1024 x 1024 x 1024 17 against 18 us and up).
+static int choose_cluster_k(int M, int N, int num_kb, int out_f32, int sms) {
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + small::TILE_N - 1) / small::TILE_N);
+  if (tiles * small::MAX_CLUSTER > (1ll << 30)) return 0;
+  if (g_cluster_k >= 0) {
+    int c = g_cluster_k >= 8 ? 8 : (g_cluster_k >= 4 ? 4 : (g_cluster_k >= 2 ? 2 : g_cluster_k));
+    while (c > 1 && num_kb < c) c /= 2;
+    return c;
+  }
+  if (tiles > sms || (out_f32 && M > BM)) return 0;
+  if (tiles * 4 <= sms) return num_kb >= 8 ? 4 : 0;
+  if (tiles * 2 <= sms) return num_kb >= 192 ? 4 : (num_kb >= 16 ? 2 : 0);
+  return num_kb >= (M <= BM ? 32 : 64) ? 2 : 0;
+}
+
 struct SyncArgs {
   const void* wait_count = nullptr;
   unsigned wait_target = 0;
@@ -901,7 +1131,12 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
     set_last_error("dh_gemm_bf16_sync: at most 8 ranks");
     return (int)cudaErrorInvalidValue;
   }
-  const int b_rows = use_pair ? pair::BN_HALF : BN;
+  const int sms = dh_sm_count();
+  const int budget = (sm_budget <= 0 || sm_budget > sms) ? sms : sm_budget;
+  const int num_kb = (K + BK - 1) / BK;
+  // the small-output kernel has one CTA per tile: no SM budget, no hooks
+  const int cluster = (mode == 0 && !hooks && sy.comm_kind == 0 && budget == sms) ? choose_cluster_k(M, N, num_kb, d_fp32, sms) : 0;
+  const int b_rows = cluster > 0 ? small::TILE_N : (use_pair ? pair::BN_HALF : BN);
   static int pair_stages = 0, pair_group = 0;
   if (pair_stages == 0) {
     const char* e = getenv("DHELLAM_GEMM_STAGES");
@@ -917,11 +1152,31 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
   const CUtensorMap* tb = b_mn_major ? get_tmap_2d(b, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, 64, BK, true)
                                      : get_tmap_2d(b, 2, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, BK, b_rows, true);
   if (!ta || !tb) return (int)cudaErrorInvalidValue;
-  const int sms = dh_sm_count();
-  int budget = (sm_budget <= 0 || sm_budget > sms) ? sms : sm_budget;
   const int sel = (a_mn_major ? 4 : 0) | (b_mn_major ? 2 : 0) | (d_fp32 ? 1 : 0);
   DeviceStatus* status = reinterpret_cast<DeviceStatus*>(dh_status_device_ptr());
 
+  if (cluster > 0) {
+    using namespace small;
+    SmallParams p;
+    p.d = d; p.ldd = ldd; p.M = M; p.N = N; p.K = K;
+    p.tiles_m = (M + BM - 1) / BM;
+    p.cluster = cluster;
+    p.accumulate = accumulate;
+    p.status = status;
+    const int tiles = p.tiles_m * ((N + TILE_N - 1) / TILE_N);
+    // one CTA per SM: a deep ring; more: two per SM, so that one's reduction and start-up run beside the other's products
+    p.stages = tiles * cluster <= sms ? MAX_STAGES : MIN_STAGES;
+    switch (sel) {
+      case 0: return launch_small<false, false, false>(ta, tb, p, tiles, stream);
+      case 1: return launch_small<false, false, true>(ta, tb, p, tiles, stream);
+      case 2: return launch_small<false, true, false>(ta, tb, p, tiles, stream);
+      case 3: return launch_small<false, true, true>(ta, tb, p, tiles, stream);
+      case 4: return launch_small<true, false, false>(ta, tb, p, tiles, stream);
+      case 5: return launch_small<true, false, true>(ta, tb, p, tiles, stream);
+      case 6: return launch_small<true, true, false>(ta, tb, p, tiles, stream);
+      default: return launch_small<true, true, true>(ta, tb, p, tiles, stream);
+    }
+  }
   if (use_pair) {
     using namespace pair;
     PairParams p;
@@ -937,7 +1192,6 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
     p.group_m = pair_group;
     p.status = status;
     const int num_tiles = p.tiles_m * p.tiles_n;
-    const int num_kb = (K + BK - 1) / BK;
     int pairs = budget / 2;
     if (pairs < 1) pairs = 1;
     p.reduce_add = accumulate ? 1 : 0;
@@ -1015,6 +1269,9 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
 // Work items per tile along K for accumulating outputs: -1 = heuristic (default; DHELLAM_GEMM_SPLITK overrides),
 // 0 / 1 = never split, n = always n (as far as K allows).
 extern "C" void dh_gemm_set_splitk(int n) { dh::gemm::g_splitk_override = n; }
+
+// Small-output kernel (128 x 128 tiles, K over a cluster): -1 = by problem (default), 0 = never, n = n CTAs per tile.
+extern "C" void dh_gemm_set_cluster_k(int n) { dh::gemm::g_cluster_k = n; }
 
 extern "C" int dh_gemm_bf16(const void* a, int64_t lda, int a_mn_major, const void* b, int64_t ldb, int b_mn_major, void* d,
                             int64_t ldd, int d_fp32, int accumulate, int M, int N, int K, int epilogue, int sm_budget,

@@ -88,6 +88,12 @@ def set_gemm_splitk(n: int):
     K.proto("dh_gemm_set_splitk", [c_int], None)(int(n))
 
 
+def set_gemm_cluster_k(n: int):
+    """Small-output kernel (128 x 128 tiles, K divided over a cluster of CTAs): -1 by problem (default), 0 never,
+    n CTAs per tile (rounded down to 1, 2, 4 or 8)."""
+    K.proto("dh_gemm_set_cluster_k", [c_int], None)(int(n))
+
+
 def gemm_nt(x, w, out=None, sm_budget: int = 0, stream=None, out_dtype=None, sync: "GemmSync | None" = None):
     """``x [M,K] @ w[N,K]ᵀ -> [M,N]``.  ``sync`` adds the collective hooks (GPU only)."""
     M, Kd = x.shape

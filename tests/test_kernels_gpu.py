@@ -112,6 +112,32 @@ def test_gemm_sm_budget_and_strided_output(gemm_mode):
     assert float(big[:, 768:].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("M,N,Kd", [(8, 512, 64), (1, 8, 520), (129, 136, 1000), (300, 1024, 576), (128, 128, 8192)])
+@pytest.mark.parametrize("cluster", [1, 2, 4, 8])
+def test_gemm_cluster_k(M, N, Kd, cluster):
+    """The small-output kernel with K over 1 to 8 CTAs: edges of tiles in M and N, K that is no multiple of a k-block or has fewer
+    k-blocks than CTAs, all operand majors, fp32 outputs stored and accumulated, a strided output.  Only the order of fp32
+    sums differs from the reference's."""
+    from dhellam_b200.ops.gemm import gemm_nn, gemm_nt, gemm_tn_acc, set_gemm_cluster_k
+    x, w, dy = bf(M, Kd), bf(N, Kd), bf(M, N)
+    big = torch.zeros(M, N + 64, dtype=torch.bfloat16, device=DEV)
+    xt, dyt, g = bf(Kd, 8 * ((M + 7) // 8)), bf(Kd, N), torch.ones(N, 8 * ((M + 7) // 8), device=DEV)
+    set_gemm_cluster_k(cluster)
+    try:
+        gemm_nt(x, w, out=big[:, :N])
+        f = gemm_nt(x, w, out_dtype=torch.float32)
+        dx = gemm_nn(dy, w)
+        gemm_tn_acc(dyt, xt, g)
+        again = gemm_nt(x, w, out_dtype=torch.float32)
+    finally:
+        set_gemm_cluster_k(-1)
+    ref = x.double() @ w.double().t()
+    assert rel(big[:, :N], ref) < 5e-3 and float(big[:, N:].abs().max()) == 0.0
+    assert rel(f, ref) < 1e-5 and torch.equal(f, again)
+    assert rel(dx, dy.double() @ w.double()) < 5e-3
+    assert rel(g, 1 + dyt.double().t() @ xt.double()) < 1e-5
+
+
 @pytest.mark.parametrize("rows,h", [(64, 256), (300, 4096), (257, 8192), (33, 1024)])
 def test_rmsnorm(rows, h, reduction_mode):
     from dhellam_b200.ops.norm import rmsnorm_bwd, rmsnorm_fwd
