@@ -183,6 +183,32 @@ __global__ void __launch_bounds__(HT) ce_stats_kernel(const void* __restrict__ l
   }
 }
 
+// Per token, from the ranks' statistics [R, T, 4] (max, sum of exp relative to it, target logit, sum of logits): the log-sum-exp and
+// the loss, with label smoothing `smooth` over `vocab` classes (0: none).  One launch of a few microseconds where the
+// same arithmetic took 9 to 13 elementwise launches.
+__global__ void __launch_bounds__(HT) ce_combine_kernel(const float4* __restrict__ stats, int R, int T, float smooth, float vocab,
+                                                        float* __restrict__ loss, float* __restrict__ lse) {
+  const int t = blockIdx.x * HT + threadIdx.x;
+  if (t >= T) return;
+  float gmax = stats[t].x;
+  for (int r = 1; r < R; ++r) {
+    const float m = stats[(size_t)r * T + t].x;
+    gmax = (m > gmax || m != m) ? m : gmax;          // a NaN stays
+  }
+  float se = 0.f, tgt = 0.f, tot = 0.f;
+  for (int r = 0; r < R; ++r) {
+    const float4 s = stats[(size_t)r * T + t];
+    se += s.y * expf(s.x - gmax);
+    tgt += s.z;
+    tot += s.w;
+  }
+  const float l = logf(se) + gmax;
+  float ce = l - tgt;
+  if (smooth != 0.f) ce = (1.f - smooth) * ce - smooth * (tot / vocab - l);
+  lse[t] = l;
+  loss[t] = ce;
+}
+
 template <bool F32>
 __global__ void __launch_bounds__(HT) ce_grad_kernel(void* __restrict__ logits, const int* __restrict__ labels, const float* __restrict__ lse,
                                                      const float* __restrict__ gtok, int T, int Vl, long long ld, int v0,
@@ -419,6 +445,15 @@ int dh_embedding_bwd_sorted(const void* dout, const void* order, const void* sor
   embedding_bwd_sorted_kernel<<<h_grid(T, 8, sm_budget), HT, 0, s>>>((const __nv_bfloat16*)dout, (const long long*)order, (const int*)sorted_tok,
                                                                      (float*)grad, T, h, Vl, v0);
   return h_rc("dh_embedding_bwd_sorted");
+}
+int dh_ce_combine(const void* stats, int R, int T, float smooth, float vocab, void* loss, void* lse, cudaStream_t s) {
+  if (R <= 0 || T <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(stats) & 15) != 0) {
+    set_last_error_c("dh_ce_combine", "statistics must be 16-byte aligned");
+    return (int)cudaErrorInvalidValue;
+  }
+  ce_combine_kernel<<<(T + HT - 1) / HT, HT, 0, s>>>((const float4*)stats, R, T, smooth, vocab, (float*)loss, (float*)lse);
+  return h_rc("dh_ce_combine");
 }
 int dh_ce_stats(const void* logits, const void* labels, void* stats, int T, int Vl, int64_t ld, int v0, int is_f32, int sm_budget,
                 cudaStream_t s) {

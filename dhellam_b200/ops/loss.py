@@ -53,6 +53,15 @@ def _smoothing(label_smoothing: float, vocab: int) -> float:
 def ce_combine_stats(all_stats, label_smoothing: float = 0.0, vocab: int = 0):
     """``all_stats [R,T,4]`` -> ``(loss [T], lse [T])``; ``vocab`` = full vocabulary size (needed
     only with label smoothing)."""
+    if K.use_native(all_stats) and all_stats.dim() == 3 and all_stats.is_contiguous() and all_stats.dtype == torch.float32 \
+            and all_stats.data_ptr() % 16 == 0:
+        R, T, _ = all_stats.shape
+        loss = torch.empty(T, dtype=torch.float32, device=all_stats.device)
+        lse = torch.empty_like(loss)
+        fn = K.proto("dh_ce_combine", [c_void_p, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p])
+        K.check(fn(all_stats.data_ptr(), R, T, _smoothing(label_smoothing, vocab), float(vocab), loss.data_ptr(), lse.data_ptr(),
+                   K.stream_ptr()), "dh_ce_combine")
+        return loss, lse
     m = all_stats[..., 0]
     gmax = m.max(dim=0).values
     se = (all_stats[..., 1] * torch.exp(m - gmax[None])).sum(0)

@@ -410,6 +410,18 @@ def test_packed_attention_against_fp32_sequence_by_sequence(ql, kl, causal, hq, 
         assert rel(torch.cat(a), torch.cat(b)) < tol, (name, rel(torch.cat(a), torch.cat(b)))
 
 
+@pytest.mark.parametrize("R,T,smoothing", [(1, 1, 0.0), (1, 257, 0.1), (4, 1000, 0.0), (8, 33, 0.1)])
+def test_ce_combine_against_the_composed_form(R, T, smoothing):
+    """Statistics of 1 to 8 ranks -> loss and log-sum-exp; same fp32 arithmetic as the PyTorch composition (CPU), so 1e-6."""
+    from dhellam_b200.ops.loss import ce_combine_stats
+    stats = torch.randn(R, T, 4) * 3
+    stats[..., 1] = stats[..., 1].exp()
+    got = ce_combine_stats(stats.cuda(), smoothing, 4096)
+    want = ce_combine_stats(stats, smoothing, 4096)
+    for g, w in zip(got, want):
+        assert rel(g, w) < 1e-6
+
+
 def test_bounded_wait_reports_timeout_without_hanging():
     """A flag that nobody sets: the device-side wait gives up after its (short) budget and
     the host reads the status word; the context stays usable."""
