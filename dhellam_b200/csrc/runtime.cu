@@ -192,6 +192,40 @@ int dh_sm_count() {
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
+// Two small int arrays from device to host with one synchronisation of `stream` (the sequence offsets of a packed attention
+// call, where reading each tensor by itself waited for the stream twice).  The copies go through a pinned buffer of the
+// calling thread, so threads on different streams do not wait for each other; it is freed with the thread.
+// ---------------------------------------------------------------------------
+namespace dh {
+struct PinnedInts {
+  static constexpr int kInts = 4096;
+  int* p = nullptr;
+  ~PinnedInts() { if (p) cudaFreeHost(p); }
+};
+}  // namespace dh
+
+extern "C" int dh_read_ints_capacity() { return dh::PinnedInts::kInts; }
+
+extern "C" int dh_read_int_pair(const void* a, int na, const void* b, int nb, int* out, cudaStream_t stream) {
+  static thread_local dh::PinnedInts buf;
+  if (na < 0 || nb < 0 || na + nb > dh::PinnedInts::kInts) {
+    dh::set_last_error("dh_read_int_pair: %d + %d values exceed the buffer of %d", na, nb, dh::PinnedInts::kInts);
+    return (int)cudaErrorInvalidValue;
+  }
+  cudaError_t e = cudaSuccess;
+  if (buf.p == nullptr) e = cudaHostAlloc(reinterpret_cast<void**>(&buf.p), sizeof(int) * dh::PinnedInts::kInts, cudaHostAllocDefault);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(buf.p, a, sizeof(int) * na, cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(buf.p + na, b, sizeof(int) * nb, cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) {
+    dh::set_last_error("dh_read_int_pair: %s", cudaGetErrorString(e));
+    return (int)e;
+  }
+  memcpy(out, buf.p, sizeof(int) * (na + nb));
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
 // Bounded-wait self test: one thread waits (for at most `budget_cycles`) on a flag that the
 // caller controls; used to check that a wait which cannot succeed returns an error status
 // instead of hanging.

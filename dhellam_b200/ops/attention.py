@@ -151,6 +151,20 @@ def _offsets(cu):
     return [int(x) for x in (cu.tolist() if torch.is_tensor(cu) else cu)]
 
 
+def _offset_pair(cq, ck):
+    """``(_offsets(cq), _offsets(ck))``; two int32 tensors on the GPU are read with one synchronisation."""
+    if torch.is_tensor(cq) and torch.is_tensor(ck) and K.use_native(cq) and K.use_native(ck) and cq.device == ck.device \
+            and cq.device.index == torch.cuda.current_device():
+        n, m = cq.numel(), ck.numel()
+        if all(c.dtype == torch.int32 and c.dim() == 1 and c.is_contiguous() for c in (cq, ck)) and n and m \
+                and n + m <= K.proto("dh_read_ints_capacity", [])():
+            out = (c_int * (n + m))()
+            K.check(K.proto("dh_read_int_pair", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p])(
+                cq.data_ptr(), n, ck.data_ptr(), m, out, K.stream_ptr()), "dh_read_int_pair")
+            return out[:n], out[n:]
+    return _offsets(cq), _offsets(ck)
+
+
 def _uniform_length(cu):
     """Common length of the sequences described by cumulative offsets ``cu`` (starting at 0), or 0 if they differ."""
     if len(cu) < 2 or cu[0] != 0:
@@ -189,8 +203,7 @@ def pymha_varlen_fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
     The whole batch is one launch, whatever the lengths.  Attention dropout is not supported by the sm_100a kernel
     (``p_dropout`` must be 0)."""
     assert p_dropout == 0.0, "attention dropout is not implemented"
-    cq = _offsets(cu_seqlens_q)
-    ck = _offsets(cu_seqlens_k)
+    cq, ck = _offset_pair(cu_seqlens_q, cu_seqlens_k)
     b = len(cq) - 1
     if _runs_packed(q, k, cq, ck, max_seqlen_q):
         from .attention_native import attn_fwd_packed
@@ -216,8 +229,7 @@ def pymha_varlen_bwd(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k
                      softmax_scale: float | None = None, is_causal: bool = True, rng_state=None, deterministic: bool = False,
                      math_sm_count: int = 0, profiling: bool = False, stream_ptr: int = 0):
     """Backward of ``pymha_varlen_fwd`` (csrc/operators/ops.h:34-52).  Returns ``(dq, dk, dv)``."""
-    cq = _offsets(cu_seqlens_q)
-    ck = _offsets(cu_seqlens_k)
+    cq, ck = _offset_pair(cu_seqlens_q, cu_seqlens_k)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     b = len(cq) - 1
     if softmax_lse.dim() == 3 and softmax_lse.shape[:2] == (b, q.shape[1]) and _runs_packed(q, k, cq, ck, softmax_lse.shape[2]):

@@ -376,6 +376,15 @@ def test_varlen_api_with_equal_lengths_uses_strided_views_of_the_packed_tensors(
         assert rel(sb(a), r) < 1e-3
 
 
+@pytest.mark.parametrize("n,m", [(2, 2), (17, 5), (2000, 2096), (2000, 2097)])
+def test_offsets_on_the_device_are_read_as_they_are(n, m):
+    """Up to the capacity of the pinned buffer in one read, beyond it one by one; int64 and strided tensors too."""
+    from dhellam_b200.ops.attention import _offset_pair
+    a, b = torch.arange(n, dtype=torch.int32) * 3, torch.arange(m, dtype=torch.int32) * 5
+    for x, y in ((a.cuda(), b.cuda()), (a.cuda().long(), b.cuda()), (torch.stack([a, a], 1).cuda()[:, 0], b.cuda()), (a, b.cuda())):
+        assert _offset_pair(x, y) == (a.tolist(), b.tolist())
+
+
 @pytest.mark.parametrize("hq,hk", [(4, 2), (3, 1), (2, 2)])
 @pytest.mark.parametrize("ql,kl,causal", [([1, 127, 128, 129, 300], None, True), ([130, 64, 257], [130, 200, 513], True),
                                           ([65, 0, 256], [40, 7, 300], False), ([17] * 150, None, True)])
