@@ -1041,16 +1041,12 @@ extern "C" void dh_gemm_set_mode(int mode) { dh::gemm::g_gemm_mode = mode; }
 namespace dh {
 namespace gemm {
 
-// Work items per tile along K for an accumulating (atomic-add) output.  A split shortens the last wave (and fills the machine
-// when there are few tiles), but every share adds the whole output to memory once more, so the rule weighs the two:
-//   rounds of the tile loop x k-blocks of a share x 512 cycles   +   shares x output elements / 584 per cycle
-// (half of the fp32 add's traffic, at the 2.1 TB/s of output that it reaches, is not hidden behind the products), and a split has
-// to win by 2 %.  4096 tokens into 6144 x 4096: unsplit 156 us, 2 / 3 / 4 shares 164 / 180 / 202; 32768 into 1536 x 4096: 346,
-// 278 / 256 / 291; 4096 into 1024 x 1024: 36, 26 / 22 / 22.  A rule on the last wave's occupancy alone took 4, 2 and 4.
-// DHELLAM_GEMM_SPLITK = 0 / 1 turns it off, = n forces n.
+// Work items per tile along K for an accumulating (atomic-add) output: the smallest split that
+// brings the last wave's occupancy above 93 %, or 1.  DHELLAM_GEMM_SPLITK = 0 / 1 turns it off,
+// = n forces n.
 static int g_splitk_override = -1;     // dh_gemm_set_splitk: -1 = follow the environment / heuristic
 
-static int choose_split_k(int tiles, int pairs, int num_kb, double out_elems) {
+static int choose_split_k(int tiles, int pairs, int num_kb) {
   static int forced = -1;
   if (g_splitk_override >= 0) {
     int b = g_splitk_override < 1 ? 1 : g_splitk_override;
@@ -1067,14 +1063,13 @@ static int choose_split_k(int tiles, int pairs, int num_kb, double out_elems) {
   if (forced >= 1) {
     best = forced;
   } else {
-    auto cost = [&](int s) {
-      const long long items = (long long)tiles * s;
-      return (double)((items + pairs - 1) / pairs) * ((num_kb + s - 1) / s) * 512.0 + s * out_elems / 584.0;
-    };
-    double bc = cost(1) * 0.98;
-    for (int s = 2; s <= 4 && num_kb / s >= 16; ++s) {
-      const double c = cost(s);
-      if (c < bc) { bc = c; best = s; }
+    auto eff = [&](int s) { const long long it = (long long)tiles * s; return (double)it / (double)(((it + pairs - 1) / pairs) * pairs); };
+    double be = eff(1);
+    if (be < 0.93) {
+      for (int s = 2; s <= 4; ++s) {
+        const double e2 = eff(s);
+        if (e2 > be + 0.03) { be = e2; best = s; }
+      }
     }
   }
   while (best > 1 && num_kb / best < 16) --best;       // keep every share long enough to amortise its prologue
@@ -1200,7 +1195,7 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
     int pairs = budget / 2;
     if (pairs < 1) pairs = 1;
     p.reduce_add = accumulate ? 1 : 0;
-    p.split_k = accumulate ? choose_split_k(num_tiles, pairs, num_kb, (double)M * N) : 1;
+    p.split_k = accumulate ? choose_split_k(num_tiles, pairs, num_kb) : 1;
     p.kb_per_split = (num_kb + p.split_k - 1) / p.split_k;
     while (p.split_k > 1 && (p.split_k - 1) * p.kb_per_split >= num_kb) --p.split_k;   // no empty share
     p.wait_count = reinterpret_cast<const uint32_t*>(sy.wait_count);
