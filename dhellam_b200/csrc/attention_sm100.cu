@@ -15,7 +15,8 @@
 //               row's maximum has grown by more than 2^8 (any reference maximum gives the same
 //               quotient; a stale one only scales numerator and denominator)
 //   While one tile is in softmax the tensor cores work on the other.
-//   Measured, causal, 8 query heads on 2 KV heads: 32768 positions 3628 us -> 1850 us, 16384 positions 452 us (1.22 PFLOP/s);
+//   Measured, causal, 8 query heads on 2 KV heads: 32768 positions inside a training step (power-capped clocks) 3628 -> 2099 us,
+//   16384 positions alone 452 us (1.22 PFLOP/s);
 //   tensor and special-function pipes each ~66 % busy, the rest is the chain softmax -> P V -> S of one tile (two softmax
 //   warps per scheduler).  Tried and slower: steps of 64 keys with S double-buffered (an N = 64 product takes as long as an
 //   N = 128 one: 2116 against 1550 cycles per tile pair); 1/8 to 1/2 of the exponentials as a polynomial on the FMA pipe
@@ -34,7 +35,7 @@
 //   dQ: one CTA per (128 queries, batch, query head) loops over the key blocks, recomputes S
 //     and dP and accumulates dQ += dS K in TMEM (dS again as a TMEM operand).  Recomputing two
 //     products per tile pair replaces an fp32 atomic accumulation of dQ and keeps dQ reproducible.
-//   Measured (same shape, 32768): dK/dV 7833 us -> 3520 us, dQ 5326 us -> 2250 us.  The forms before ran one phase after
+//   Measured (32768 positions in the step): dK/dV 7833 -> 4071 us, dQ 5326 -> 2708 us; 16384 alone 867 and 568 us.  The forms before ran one phase after
 //   the other and applied the mask as predicates (10 ALU instructions per score in dQ).
 //
 // MMAs are issued under a predicate by a warp whose control flow stays uniform (ptx.cuh, umma_bf16_by): issued inside
