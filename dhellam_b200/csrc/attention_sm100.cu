@@ -11,9 +11,10 @@
 //   warp 0      TMA producer: Q tiles once, then K_j / V_j through one 5-slot ring
 //   warp 1      MMA issuer:   S_t = Q_t K_j^T, O_t += P_t V_j (t = 0, 1) with P read from TMEM
 //   warps 4-7, 8-11  softmax of tile 0 / 1: one thread per row, no exchange between threads; P_t
-//               overwrites S_t in TMEM as bf16; O_t stays in TMEM and is rescaled only when a
-//               row's maximum has grown by more than 2^8 (any reference maximum gives the same
-//               quotient; a stale one only scales numerator and denominator)
+//               overwrites S_t in TMEM as bf16; O_t stays in TMEM and is rescaled when the maximum
+//               of one of the warp's rows has grown.  (Keeping a maximum until it has grown by a
+//               factor, as published for flash attention on this hardware, is faster but less exact:
+//               the largest probability of a row is then rounded to bf16 where it would be exactly 1.)
 //   While one tile is in softmax the tensor cores work on the other.
 //   Measured, causal, 8 query heads on 2 KV heads: 32768 positions inside a training step (power-capped clocks) 3628 -> 2099 us,
 //   16384 positions alone 452 us (1.22 PFLOP/s);
@@ -197,7 +198,6 @@ struct FwdCtl {
   int abort_flag;
 };
 constexpr int FWD_SMEM = TILE_BYTES * (2 + FWD_RING) + 1024 + 512;
-constexpr float RESCALE_LOG2 = 8.f;          // P stays below 2^8: as exact in bf16 as below 1
 
 struct FwdArgs {
   __nv_bfloat16* out;
@@ -365,24 +365,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         for (int c = 0; c < 4; ++c) mx[c] = fmaxf(mx[c], __uint_as_float(s[i + c]));
       }
       const float bm = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      if (j == 0) {
-        m = bm;
-      } else if (__any_sync(0xffffffffu, (bm - m) * sl2 > RESCALE_LOG2)) {
+      // every new maximum becomes the reference at once: the largest probability is then exactly 1 and loses nothing in bf16
+      const bool grown = j > 0 && __any_sync(0xffffffffu, bm > m);
+      float alpha = 1.f;
+      if (grown) {
         // a reference of -inf (nothing seen yet) has zero sums: any factor will do, 0 is finite
         const float m_new = fmaxf(m, bm);
-        const float alpha = m == -INFINITY ? 0.f : ex2((m - m_new) * sl2);
+        alpha = m == -INFINITY ? 0.f : ex2((m - m_new) * sl2);
         m = m_new;
         l2 = mul2(l2, pk2(alpha, alpha));
-        // S_t(j) was issued behind P V of block j - 1, so O_t is complete up to that block
-#pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-          uint32_t o[16];
-          tmem_ld16(to + c * 16, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st16(to + c * 16, o);
-        }
+      } else if (j == 0) {
+        m = bm;
       }
       const float nm = m == -INFINITY ? 0.f : -m * sl2;
       const uint64_t nm2 = pk2(nm, nm);
@@ -402,6 +395,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
             p[i] = pack_bf16x2(x, y);
           }
           tmem_st8(ts + c * 8, p);
+        }
+        if (h == 0 && grown) {
+          // S_t(j) was issued behind P V of block j - 1, so O_t is complete up to that block, and the next P V waits for p_ready.
+          // Here half of the scores' registers are free: 32 columns to a round trip (16384 positions, 8 heads on 2: 473 us; in
+          // front of the exponentials, 16 to a round trip, 518; 432 if a growth below 2^8 is let pass)
+#pragma unroll 1
+          for (int c = 0; c < D; c += 32) {
+            uint32_t o[2][16];
+            tmem_ld16(to + c, o[0]);
+            tmem_ld16(to + c + 16, o[1]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i >> 4][i & 15] = __float_as_uint(__uint_as_float(o[i >> 4][i & 15]) * alpha);
+            tmem_st16(to + c, o[0]);
+            tmem_st16(to + c + 16, o[1]);
+          }
         }
         tmem_st_wait();
         tc_fence_before();

@@ -337,6 +337,59 @@ def test_attention_large_shapes_against_fp32(Sq, Sk, B, Hq, Hk):
     assert rel(dv, vf.grad) < 2e-2, ("dv", rel(dv, vf.grad))
 
 
+def _peaked_scores(kind, Sq, Sk, Hq, Hk):
+    """Inputs whose softmax has few dominant keys, as trained models have: scores with a standard deviation of 3 or 6, scores
+    that rise with the key index (every key block has a new maximum), one key that outgrows the others by more than 2^8."""
+    d = 128
+    q, k, v = bf(Sq, 1, Hq, d), bf(Sk, 1, Hk, d), bf(Sk, 1, Hk, d)
+    if kind in ("std3", "std6"):
+        q *= float(kind[3:])
+    elif kind == "rising":
+        k[:, :, :, 0] = torch.linspace(-8, 8, Sk, device=DEV)[:, None, None].to(torch.bfloat16)
+        q[:, :, :, 0] = 12.0
+    else:
+        k[Sk // 2] = 40.0 * q[Sq // 2, :, :Hk] / q[Sq // 2, :, :Hk].float().norm(dim=-1, keepdim=True)
+    return q, k, v
+
+
+def _running_maximum_reference(q, k, v, causal, scale):
+    """``(out, lse, out as flash attention rounds it)`` in 64 bits: the third divides sums whose probabilities are rounded to
+    bf16 relative to the running maximum of blocks of 128 keys, the only rounding of a forward pass besides that of its result."""
+    Sq, Hq, Sk = q.shape[0], q.shape[2], k.shape[0]
+    g = Hq // k.shape[2]
+    qd, kd, vd = (t[:, 0].transpose(0, 1).double() for t in (q, k, v))
+    kd, vd = kd.repeat_interleave(g, 0), vd.repeat_interleave(g, 0)
+    s = qd @ kd.transpose(1, 2) * scale
+    if causal:
+        s.masked_fill_(torch.arange(Sk, device=DEV)[None] > torch.arange(Sq, device=DEV)[:, None] + (Sk - Sq), float("-inf"))
+    lse = torch.logsumexp(s, -1)
+    exact = torch.softmax(s, -1) @ vd
+    pad = -Sk % 128
+    s = torch.nn.functional.pad(s, (0, pad), value=float("-inf")).view(Hq, Sq, -1, 128)
+    run = s.amax(-1).cummax(-1).values
+    p = torch.exp(s - run[..., None])
+    w = torch.exp(run - run[..., -1:])[..., None]
+    num = (p.to(torch.bfloat16).double() * w).view(Hq, Sq, -1)[..., :Sk] @ vd
+    rounded = (num / (p * w).sum((-1, -2))[..., None]).to(torch.bfloat16)
+    back = lambda t: t.transpose(0, 1).unsqueeze(1)
+    return back(exact), lse.unsqueeze(0), back(rounded)
+
+
+@pytest.mark.parametrize("Sq,Sk,Hq,Hk,causal", [(1024, 1024, 4, 2, True), (300, 2000, 3, 1, False)])
+@pytest.mark.parametrize("kind", ["std3", "std6", "rising", "spike"])
+def test_attention_forward_is_as_exact_as_the_running_maximum_allows(kind, Sq, Sk, Hq, Hk, causal):
+    """Against 64 bits, the forward is no further off than what the rounding of probabilities below the running maximum and of the
+    result costs (computed beside it; 3 % for the 32-bit arithmetic and for sums in another order)."""
+    from dhellam_b200.ops.attention import attn_fwd
+    q, k, v = _peaked_scores(kind, Sq, Sk, Hq, Hk)
+    scale = 1.0 / math.sqrt(128)
+    out, lse = attn_fwd(q, k, v, causal, scale)
+    exact, exact_lse, rounded = _running_maximum_reference(q, k, v, causal, scale)
+    off = lambda t: ((t.double() - exact).norm() / exact.norm()).item()
+    assert off(out) < 1.03 * off(rounded), (off(out), off(rounded))
+    assert (lse.double() - exact_lse).abs().max().item() < 1e-4 * (1 + exact_lse.abs().max().item())
+
+
 @pytest.mark.parametrize("budget", [1, 5, 24, 100])
 def test_attention_sm_budget_gives_identical_results(budget):
     """With an SM budget the attention kernels run as consecutive launches of at most that many CTAs
