@@ -206,7 +206,9 @@ struct FwdArgs {
   int head_pair;                             // 1: a CTA's two tiles are query heads 2h, 2h+1; 0: row tiles 2i, 2i+1 of one head
 };
 
-template <class Table>
+// POSITIVE: the scale is; a form of its own for the others, whose masked keys need more than a score of -inf (as one
+// kernel 3 % slower for everybody).
+template <class Table, bool POSITIVE>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                 const __grid_constant__ Geometry g, const __grid_constant__ FwdArgs a, const __grid_constant__ Table table) {
@@ -378,7 +380,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         m = bm;
       }
       const float nm = m == -INFINITY ? 0.f : -m * sl2;
-      const uint64_t nm2 = pk2(nm, nm);
+      uint64_t mul = sl2_2, add = pk2(nm, nm);
+      if (!POSITIVE && !full) {
+        // -inf times the scale is -inf only for a positive one: the exponents of masked keys are set here instead
+#pragma unroll
+        for (int i = 0; i < BKV; ++i) s[i] = __float_as_uint(i < limit ? fmaf(__uint_as_float(s[i]), sl2, nm) : -INFINITY);
+        mul = pk2(1.f, 1.f);
+        add = 0;
+      }
       uint64_t rs[2] = {0, 0};                       // the block's own sum: short chains, then one add to the running sum
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -389,7 +398,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
           for (int i = 0; i < 8; ++i) {
             const int e = c * 16 + 2 * i;
             float x, y;
-            upk2(fma2(pk2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sl2_2, nm2), x, y);
+            upk2(fma2(pk2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), mul, add), x, y);
             x = ex2(x); y = ex2(y);
             rs[i & 1] = add2(rs[i & 1], pk2(x, y));
             p[i] = pack_bf16x2(x, y);
@@ -1188,7 +1197,8 @@ template <class Table>
 static void run_fwd(const FwdMaps& m, Geometry& g, const FwdArgs& a, const Table& table, long long items, int sm_budget, cudaStream_t stream) {
   launch_in_waves(items, sm_budget, [&](unsigned n, int x0) {
     g.x0 = x0;
-    attn_fwd_kernel<Table><<<n, THREADS, FWD_SMEM, stream>>>(*m.q, *m.k, *m.v, g, a, table);
+    if (g.scale > 0.f) attn_fwd_kernel<Table, true><<<n, THREADS, FWD_SMEM, stream>>>(*m.q, *m.k, *m.v, g, a, table);
+    else attn_fwd_kernel<Table, false><<<n, THREADS, FWD_SMEM, stream>>>(*m.q, *m.k, *m.v, g, a, table);
   });
 }
 
@@ -1251,8 +1261,9 @@ static void run_dq(const BwdMaps& m, Geometry& g, const DqArgs& a, const Table& 
 }
 template <class Table>
 static cudaError_t opt_in_fwd() {
-  static PerDeviceFlags done;
-  return opt_in(attn_fwd_kernel<Table>, FWD_SMEM, done);
+  static PerDeviceFlags done, done_other;
+  cudaError_t e = opt_in(attn_fwd_kernel<Table, true>, FWD_SMEM, done);
+  return e != cudaSuccess ? e : opt_in(attn_fwd_kernel<Table, false>, FWD_SMEM, done_other);
 }
 template <class Table>
 static cudaError_t opt_in_bwd() {

@@ -390,6 +390,24 @@ def test_attention_forward_is_as_exact_as_the_running_maximum_allows(kind, Sq, S
     assert (lse.double() - exact_lse).abs().max().item() < 1e-4 * (1 + exact_lse.abs().max().item())
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+def test_attention_with_a_scale_that_is_not_positive(scale):
+    """Masked keys stay masked whatever the sign of the scale: with 0 every visible key weighs the same.  Ragged and causal, so
+    that there are masked keys in the last tile of the keys and on the diagonal."""
+    from dhellam_b200.ops.attention import attn_bwd, attn_fwd
+    S, d = 200, 128
+    q, k, v, do = bf(S, 2, 2, d), bf(S, 2, 1, d), bf(S, 2, 1, d), bf(S, 2, 2, d)
+    cpu = lambda *ts: [t.cpu().float() for t in ts]
+    for causal in (True, False):
+        o, lse = attn_fwd(q, k, v, causal, scale)
+        oref, lref = attn_fwd(*cpu(q, k, v), causal, scale)
+        assert rel(o, oref) < 1e-2 and rel(lse, lref) < 1e-3
+        grads = attn_bwd(do, q, k, v, o, lse, causal, scale)
+        refs = attn_bwd(*cpu(do, q, k, v), oref, lref, causal, scale)
+        for a, r in zip(grads, refs):
+            assert (a.cpu().float() - r).norm() <= 2e-2 * r.norm()       # dq and dk are zero at scale 0
+
+
 @pytest.mark.parametrize("budget", [1, 5, 24, 100])
 def test_attention_sm_budget_gives_identical_results(budget):
     """With an SM budget the attention kernels run as consecutive launches of at most that many CTAs
