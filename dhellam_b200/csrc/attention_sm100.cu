@@ -141,10 +141,6 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, ui
   tma_load_4d(dst, m, bar, 0, head, b, row);
   tma_load_4d(dst + HALF_BYTES, m, bar, 64, head, b, row);
 }
-// Bounded wait of a whole warp with one answer for all lanes, so that the control flow behind it stays uniform.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, DeviceStatus* st, int where) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, st, where));
-}
 // Zeroes rows [first, 128) of a tile in shared memory (whole warp); a row is 128 bytes in each of the two boxes.
 __device__ __forceinline__ void zero_tile_rows(uint8_t* tile, int first, int lane) {
   for (int h = 0; h < 2; ++h)
@@ -346,7 +342,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     uint64_t l2 = pk2(0.f, 0.f);                     // row sum in two interleaved parts
     bool ok = nblk > 0;
     for (int j = 0; j < nblk && ok; ++j) {
-      if (!mbar_wait(&ctl->s_full[t], j & 1, abort_flag, g.status, 420)) { ok = false; break; }
+      if (!warp_wait(&ctl->s_full[t], j & 1, abort_flag, g.status, 420)) { ok = false; break; }
       tc_fence_after();
       const int limit = visible_keys(w.nk, g.causal, off, qi, j * BKV);
       const bool full = __all_sync(0xffffffffu, limit >= BKV);
@@ -434,7 +430,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     __nv_bfloat16* orow = a.out + (long long)(w.q0 + qi) * a.o_s + (long long)w.b * a.o_b + (long long)hq_[t] * a.o_h;
     float* lrow = a.lse + ((long long)w.sid * g.Hq + hq_[t]) * g.ls + qi;
     if (nblk > 0) {
-      if (ok && mbar_wait(&ctl->o_done[t], 0, abort_flag, g.status, 422)) {
+      if (ok && warp_wait(&ctl->o_done[t], 0, abort_flag, g.status, 422)) {
         tc_fence_after();
         const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
@@ -702,7 +698,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         L[i] = q < w.nq ? -lp[q] * LOG2E : -INFINITY;
         dl[i] = q < w.nq ? -dp[q] : 0.f;
       }
-      if (!mbar_wait(&ctl->stat_empty[st], ph, abort_flag, g.status, 515)) break;
+      if (!warp_wait(&ctl->stat_empty[st], ph, abort_flag, g.status, 515)) break;
       float* dst = sStat + st * 2 * BQ;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -732,8 +728,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       const bool edge = (qb + 1) * BQ > w.nq || (kb + 1) * BKV > w.nk || (g.causal && kb * BKV + BKV - 1 > qb * BQ + off);
       const int lo = kj >= w.nk ? BQ : (g.causal ? kj - off - qbase : 0);
       const int hi = w.nq - qbase;
-      if (!mbar_wait(&ctl->stat_full[sst], (it / STAT_RING) & 1, abort_flag, g.status, 520)) { ok = false; break; }
-      if (!mbar_wait(&ctl->s_full, it & 1, abort_flag, g.status, 521)) { ok = false; break; }
+      if (!warp_wait(&ctl->stat_full[sst], (it / STAT_RING) & 1, abort_flag, g.status, 520)) { ok = false; break; }
+      if (!warp_wait(&ctl->s_full, it & 1, abort_flag, g.status, 521)) { ok = false; break; }
       tc_fence_after();
       // the mask is a path of its own: as predicates it costs more issue slots than the arithmetic
       uint64_t p[32];
@@ -772,7 +768,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       };
       if (edge) probabilities(std::true_type{});
       else probabilities(std::false_type{});
-      if (!mbar_wait(&ctl->dp_full, it & 1, abort_flag, g.status, 522)) { ok = false; break; }
+      if (!warp_wait(&ctl->dp_full, it & 1, abort_flag, g.status, 522)) { ok = false; break; }
       tc_fence_after();
       {
         uint32_t v[64];
@@ -813,7 +809,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     __nv_bfloat16* dvr = a.dv + krow * a.dv_s + (long long)w.b * a.dv_b + (long long)hk * a.dv_h + half * 64;
     __nv_bfloat16* dkr = a.dk + krow * a.dk_s + (long long)w.b * a.dk_b + (long long)hk * a.dk_h + half * 64;
     if (n_iter > 0) {
-      if (ok && mbar_wait(&ctl->acc_full, 0, abort_flag, g.status, 523)) {
+      if (ok && warp_wait(&ctl->acc_full, 0, abort_flag, g.status, 523)) {
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
@@ -1020,7 +1016,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       int limit = visible_keys(w.nk, g.causal, off, qi, j * BKV + half * 64);
       if (!row_ok) limit = 0;
       const bool full = __all_sync(0xffffffffu, limit >= 64);
-      if (!mbar_wait(&ctl->s_full[j & 1], (j >> 1) & 1, abort_flag, g.status, 820)) { ok = false; break; }
+      if (!warp_wait(&ctl->s_full[j & 1], (j >> 1) & 1, abort_flag, g.status, 820)) { ok = false; break; }
       tc_fence_after();
       auto gradients = [&](auto edge_) -> bool {       // as in the dK/dV kernel, the mask is a path of its own
         constexpr bool masked = decltype(edge_)::value;
@@ -1037,7 +1033,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             p[c * 16 + i] = pk2(ex2(x), ex2(y));
           }
         }
-        if (!mbar_wait(&ctl->dp_full, j & 1, abort_flag, g.status, 821)) return false;
+        if (!warp_wait(&ctl->dp_full, j & 1, abort_flag, g.status, 821)) return false;
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -1068,7 +1064,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     }
     __nv_bfloat16* dqr = a.dq + (long long)(w.q0 + qi) * a.dq_s + (long long)w.b * a.dq_b + (long long)hq * a.dq_h + half * 64;
     if (nblk > 0) {
-      if (ok && mbar_wait(&ctl->dq_full, 0, abort_flag, g.status, 822)) {
+      if (ok && warp_wait(&ctl->dq_full, 0, abort_flag, g.status, 822)) {
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {

@@ -248,7 +248,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       int tm, tn;
       tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-      if (!mbar_wait(&ctl->acc_full[acc], acc_ph, abort_flag, p.status, 300)) { ok = false; break; }
+      if (!warp_wait(&ctl->acc_full[acc], acc_ph, abort_flag, p.status, 300)) { ok = false; break; }
       tc_fence_after();
       const int row = tm * BM + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
@@ -598,11 +598,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const Item im = item_coords(it, p, num_tiles, num_kb);
         const int kb0 = im.kb0, kb1 = im.kb1;
         if (kb0 >= kb1) continue;                       // an expert without rows: nothing to add (all roles skip the item)
-        if (!__all_sync(0xffffffffu, mbar_wait<true>(&ctl->acc_empty[acc], acc_ph ^ 1, abort_flag, p.status, 210, p.wait_budget))) { ok = false; break; }
+        if (!warp_wait<true>(&ctl->acc_empty[acc], acc_ph ^ 1, abort_flag, p.status, 210, p.wait_budget)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * ACC_COLS;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&ctl->full[s], ph, abort_flag, p.status, 211, p.wait_budget))) { ok = false; break; }
+          if (!warp_wait(&ctl->full[s], ph, abort_flag, p.status, 211, p.wait_budget)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_base = smem_u32(sA + s * A2_STAGE_BYTES);
           const uint32_t b_base = smem_u32(sB + s * B2_STAGE_BYTES);
@@ -701,7 +701,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const Item im = item_coords(it, p, num_tiles, num_kb);
       const int tm = im.tm, tn = im.tn;
       if (im.kb0 >= im.kb1) continue;
-      if (!mbar_wait(&ctl->acc_full[acc], acc_ph, abort_flag, p.status, 310, p.wait_budget)) { ok = false; break; }
+      if (!warp_wait(&ctl->acc_full[acc], acc_ph, abort_flag, p.status, 310, p.wait_budget)) { ok = false; break; }
       tc_fence_after();
       const int row0 = tm * TILE_M + (int)rank * BM + quarter * 32;     // first of this warp's 32 output rows
       const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
@@ -915,7 +915,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     uint32_t ph = 0;
     bool ok = true;
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&ctl->full[s], ph, abort_flag, p.status, 220))) { ok = false; break; }
+      if (!warp_wait(&ctl->full[s], ph, abort_flag, p.status, 220)) { ok = false; break; }
       tc_fence_after();
       const uint32_t a_base = smem_u32(smem + s * SLOT_BYTES), b_base = a_base + A_BYTES;
 #pragma unroll
@@ -931,7 +931,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else {
     // partial tile -> this CTA's shared memory (all loads have landed and all products have read them)
     const int quarter = warp & 3;
-    if (mbar_wait(&ctl->done, 0, abort_flag, p.status, 320)) {
+    if (warp_wait(&ctl->done, 0, abort_flag, p.status, 320)) {
       tc_fence_after();
       float* row = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * ACC_LD;
 #pragma unroll 1

@@ -128,6 +128,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Bounded wait of a whole warp with one answer for all lanes.  Lanes poll for themselves, so without the vote a barrier that
+// completes just as the wait gives up would send some lanes on and others out of the loop, and the ones that go on would
+// never be joined in the warp-wide instructions behind it (votes, TMEM loads and stores).
+template <bool kCluster = false>
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, DeviceStatus* st, int where,
+                                          long long budget = DH_WAIT_BUDGET_CYCLES) {
+  return __all_sync(0xffffffffu, mbar_wait<kCluster>(bar, parity, abort_flag, st, where, budget));
+}
+
 // ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies).  Every CTA fetches its own tiles.
 // The innermost coordinate times the element size must be a multiple of 16 bytes.
