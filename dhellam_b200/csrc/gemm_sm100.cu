@@ -947,7 +947,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
   __syncwarp();
   cluster_sync_all();                      // all partial tiles of the cluster are in place
-  {
+  uint32_t gave_up = 0;                    // a CTA whose wait ran out has no partial tile: the output then stays as it was
+#pragma unroll
+  for (int k = 0; k < MAX_CLUSTER; ++k)
+    if (k < p.cluster) gave_up |= ld_cluster_u32(mapa_u32(smem_u32(&ctl->abort_flag), (uint32_t)k));
+  if (gave_up == 0) {
     // row i of this CTA's share: a warp per row, four columns per lane
     const int rows = BM / p.cluster;
     const int col = n0 + 4 * lane;
