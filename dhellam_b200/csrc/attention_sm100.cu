@@ -1317,6 +1317,8 @@ static Geometry geometry(int B, int Hq, int Hk, int Sq, int Sk, int Tq, int Tk, 
   g.status = reinterpret_cast<DeviceStatus*>(dh_status_device_ptr());
   return g;
 }
+constexpr long long MAX_BWD_ROWS = 1ll << 26;       // query rows x heads (x batch) of one dense backward, or of one sequence
+
 static bool heads_ok(const char* who, int d, int Hq, int Hk) {
   if (d != D) { set_last_error("%s: head size %d is not supported (128 only)", who, d); return false; }
   if (Hk <= 0 || Hq % Hk != 0) { set_last_error("%s: query heads must be a multiple of KV heads", who); return false; }
@@ -1408,7 +1410,7 @@ int dh_attn_bwd(const void* dout, const void* q, const void* k, const void* v, c
   cudaError_t e = opt_in_bwd<Dense>();
   if (e != cudaSuccess) return (int)e;
   const long long rows_ll = (long long)B * Hq * Sq;
-  if (rows_ll > (1ll << 26)) {     // statistics are indexed well inside 32 bits
+  if (rows_ll > MAX_BWD_ROWS) {
     set_last_error("dh_attn_bwd: B*Hq*Sq = %lld rows exceed the supported 2^26", rows_ll);
     return (int)cudaErrorInvalidValue;
   }
@@ -1425,9 +1427,12 @@ int dh_attn_bwd_packed(const void* dout, const void* q, const void* k, const voi
   if (nseq <= 0 || Tq <= 0 || Tk <= 0) return 0;
   const Sequences seqs = {nseq, cu_q, cu_k};
   if (!offsets_ok("dh_attn_bwd_packed", seqs, Tq, Tk, lse_rows)) return (int)cudaErrorInvalidValue;
-  if ((long long)Hq * Tq > (1ll << 26)) {
-    set_last_error("dh_attn_bwd_packed: %lld query rows exceed the supported 2^26", (long long)Hq * Tq);
-    return (int)cudaErrorInvalidValue;
+  for (int i = 0; i < nseq; ++i) {
+    const long long rows = (long long)Hq * (cu_q[i + 1] - cu_q[i]);
+    if (rows > MAX_BWD_ROWS) {
+      set_last_error("dh_attn_bwd_packed: Hq*Sq = %lld rows of sequence %d exceed the supported 2^26", rows, i);
+      return (int)cudaErrorInvalidValue;
+    }
   }
   const int64_t* sdo = strides; const int64_t* sq = strides + 3; const int64_t* sk = strides + 6; const int64_t* sv = strides + 9;
   const BwdMaps m = {tensor_map_sbhd(q, Tq, 1, Hq, sq[0], sq[0], sq[2]), tensor_map_sbhd(k, Tk, 1, Hk, sk[0], sk[0], sk[2]),

@@ -1,0 +1,60 @@
+"""What the packed attention entry points accept and refuse before they launch anything (CPU)."""
+import ctypes
+from ctypes import c_float, c_int, c_int64, c_void_p
+
+import pytest
+
+import pytest
+import torch
+
+from dhellam_b200 import kernels as K
+
+
+def _backward_with(lengths, heads):
+    """Error text of a packed backward over null operands: the operands are the last thing that is looked at before a launch."""
+    cu = [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    off = (c_int * len(cu))(*cu)
+    p_int = ctypes.POINTER(c_int)
+    fn = K.proto("dh_attn_bwd_packed", [c_void_p] * 10 + [ctypes.POINTER(c_int64), c_int, p_int, p_int, c_int, c_int, c_int, c_int, c_int,
+                                                          c_int, c_int, c_float, c_int, c_void_p])
+    rc = fn(*[0] * 10, (c_int64 * 24)(*[heads * 128, heads * 128, 128] * 8), len(lengths), off, off, cu[-1], cu[-1], max(lengths), heads,
+            heads, 128, 1, 1.0, 0, 0)
+    assert rc != 0
+    return K.lib().dh_last_error_string().decode()
+
+
+def test_the_row_limit_of_the_backward_holds_per_sequence():
+    """64 heads and 2^21 tokens in documents of unequal length: 2^27 rows in all, at most 2^25 in one sequence."""
+    lengths = [2 ** 19, 2 ** 19 - 7, 2 ** 18, 2 ** 19, 2 ** 18 + 7]
+    assert 64 * sum(lengths) > 2 ** 26 > 64 * max(lengths)
+    assert "2^26" not in _backward_with(lengths, 64)
+    assert "2^26" in _backward_with([2 ** 20 + 1, 5], 64)
+
+
+def _operands(tq=50, tk=50):
+    bf = lambda t, h: torch.zeros(t, h, 128, dtype=torch.bfloat16)
+    return dict(q=bf(tq, 2), k=bf(tk, 1), v=bf(tk, 1), dout=bf(tq, 2), out=bf(tq, 2), lse=torch.zeros(2, 2, 30),
+                dq=bf(tq, 2), dk=bf(tk, 1), dv=bf(tk, 1))
+
+
+BAD = {"fp16": lambda t: t.half(), "fp32": lambda t: t.double() if t.dtype == torch.float32 else t.float(), "short": lambda t: t[:49],
+       "heads": lambda t: t.repeat(1, 2, 1), "columns": lambda t: t.transpose(1, 2).contiguous().transpose(1, 2).repeat(1, 1, 1)[:, :, ::2]}
+
+
+@pytest.mark.parametrize("how", BAD)
+@pytest.mark.parametrize("which", ["q", "k", "v", "dout", "out", "lse"])
+def test_operands_that_the_kernels_would_misread_are_refused(which, how):
+    """Other types, too few rows, other heads or strided columns: the kernels see addresses and strides only."""
+    from dhellam_b200.ops.attention_native import attn_bwd_packed, attn_fwd_packed
+    if which == "lse" and how in ("short", "heads", "columns"):
+        pytest.skip("the caller checks its shape")
+    o = _operands()
+    o[which] = BAD[how](o[which])
+    cu = [0, 20, 50]
+    if which in ("q", "k", "v") and not (which == "q" and how == "heads"):     # four query heads on one KV head are fine
+        with pytest.raises(AssertionError):
+            attn_fwd_packed(o["q"], o["k"], o["v"], cu, cu, 30, True, None)
+    with pytest.raises(AssertionError):
+        attn_bwd_packed(o["dout"], o["q"], o["k"], o["v"], o["out"], o["lse"], o["dq"], o["dk"], o["dv"], cu, cu, True, None)
