@@ -50,37 +50,49 @@ def _packed_offsets(cu):
     return (c_int * len(cu))(*cu)
 
 
+def _packed_strides(operands, d, device):
+    """``(row, head)`` strides of ``(tensor, heads)`` pairs.  The kernels see addresses and strides only: that these are bf16 rows of
+    ``[T, heads, d]`` on one device is made sure of here."""
+    strides = []
+    for t, heads in operands:
+        _, h, c = t.shape
+        row, head, column = t.stride()
+        assert h == heads and c == d and column == 1 and t.dtype == torch.bfloat16 and t.get_device() == device
+        strides.append((row, head))
+    return strides
+
+
 def attn_fwd_packed(q, k, v, cq, ck, max_q, causal, scale, sm_budget=0, stream=None):
-    """Packed batch in one launch: ``q [Tq, Hq, d]``, ``k, v [Tk, Hk, d]``, offsets as Python lists (checked by the
-    caller).  Returns ``(out like q, lse [b, Hq, max_q])``; statistics past a sequence's end are ``-inf``."""
+    """Packed batch in one launch: ``q [Tq, Hq, d]``, ``k, v [Tk, Hk, d]``, offsets as Python lists that ascend (checked by
+    the caller); rows past the last sequence are not looked at.  Returns ``(out like q, lse [b, Hq, max_q])``; statistics past a
+    sequence's end are ``-inf``."""
     Tq, Hq, d = q.shape
-    Tk, Hk = k.shape[0], k.shape[1]
-    assert q.stride(2) == 1 and k.stride(2) == 1 and v.stride(2) == 1
-    scale = scale if scale is not None else 1.0 / math.sqrt(d)
+    Tk, Hk = min(k.shape[0], v.shape[0]), k.shape[1]
     out = torch.empty_like(q)
-    assert out.stride(2) == 1
+    strides = _packed_strides(((q, Hq), (k, Hk), (v, Hk), (out, Hq)), d, q.get_device())
+    assert cq[-1] <= Tq and ck[-1] <= Tk
+    scale = scale if scale is not None else 1.0 / math.sqrt(d)
     b = len(cq) - 1
     whole = all(cq[i + 1] - cq[i] == max_q for i in range(b))
     shape = (b, Hq, max_q)
     lse = torch.empty(shape, dtype=torch.float32, device=q.device) if whole else \
         torch.full(shape, float("-inf"), dtype=torch.float32, device=q.device)
-    strides = (c_int64 * 8)(*(s for t in (q, k, v, out) for s in (t.stride(0), t.stride(1))))
     fn = K.proto("dh_attn_fwd_packed", [c_void_p] * 5 + [ctypes.POINTER(c_int64), c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int),
                                                          c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
-    K.check(fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), strides, b, _packed_offsets(cq),
-               _packed_offsets(ck), Tq, Tk, max_q, Hq, Hk, d, 1 if causal else 0, scale, sm_budget, K.stream_ptr(stream)),
-            "dh_attn_fwd_packed")
+    K.check(fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), (c_int64 * 8)(*(s for p in strides for s in p)), b,
+               _packed_offsets(cq), _packed_offsets(ck), Tq, Tk, max_q, Hq, Hk, d, 1 if causal else 0, scale, sm_budget,
+               K.stream_ptr(stream)), "dh_attn_fwd_packed")
     return out, lse
 
 
 def attn_bwd_packed(dout, q, k, v, out, lse, dq, dk, dv, cq, ck, causal, scale, sm_budget=0, stream=None):
     """Backward of ``attn_fwd_packed`` into ``dq, dk, dv``."""
-    Tq, Hq, d = q.shape
-    Tk, Hk = k.shape[0], k.shape[1]
+    Hq, d, Hk, device = q.shape[1], q.shape[2], k.shape[1], q.get_device()
     strides = []
-    for t in (dout, q, k, v, out, dq, dk, dv):
-        assert t.stride(2) == 1 and t.dtype == torch.bfloat16
-        strides += [t.stride(0), t.stride(0), t.stride(1)]
+    for row, head in _packed_strides(((dout, Hq), (q, Hq), (k, Hk), (v, Hk), (out, Hq), (dq, Hq), (dk, Hk), (dv, Hk)), d, device):
+        strides += (row, row, head)
+    Tq, Tk = min(t.shape[0] for t in (q, dout, out, dq)), min(t.shape[0] for t in (k, v, dk, dv))
+    assert cq[-1] <= Tq and ck[-1] <= Tk and lse.dtype == torch.float32 and lse.get_device() == device
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
     lse = lse.contiguous()
     b = len(cq) - 1

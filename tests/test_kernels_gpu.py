@@ -490,6 +490,19 @@ def test_packed_attention_against_fp32_sequence_by_sequence(ql, kl, causal, hq, 
         assert rel(torch.cat(a), torch.cat(b)) < tol, (name, rel(torch.cat(a), torch.cat(b)))
 
 
+def test_packed_attention_with_operands_of_different_lengths():
+    """Operands may hold rows past the last sequence, each as many as it likes."""
+    from dhellam_b200.ops.attention import pymha_varlen_bwd, pymha_varlen_fwd
+    cu, n = [0, 200, 333], 333
+    q, k, v, do = bf(n + 3, 4, 128), bf(n, 2, 128), bf(n + 130, 2, 128), bf(n + 1, 4, 128)
+    long_out, long_lse = pymha_varlen_fwd(q, k, v, cu, cu, 200, 200)
+    longs = (long_out, long_lse, *pymha_varlen_bwd(do, q, k, v, long_out, long_lse, cu, cu, 200, 200))
+    out, lse = pymha_varlen_fwd(q[:n], k, v[:n], cu, cu, 200, 200)
+    shorts = (out, lse, *pymha_varlen_bwd(do[:n], q[:n], k, v[:n], out, lse, cu, cu, 200, 200))
+    for i, (a, b) in enumerate(zip(longs, shorts)):
+        assert torch.equal(a if i == 1 else a[:n], b)
+
+
 @pytest.mark.parametrize("R,T,smoothing", [(1, 1, 0.0), (1, 257, 0.1), (4, 1000, 0.0), (8, 33, 0.1)])
 def test_ce_combine_against_the_composed_form(R, T, smoothing):
     """Statistics of 1 to 8 ranks -> loss and log-sum-exp; same fp32 arithmetic as the PyTorch composition (CPU), so 1e-6."""
