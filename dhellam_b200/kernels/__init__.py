@@ -12,6 +12,7 @@ from ctypes import c_char_p, c_float, c_int, c_int64, c_uint64, c_void_p
 from pathlib import Path
 
 import torch
+from torch.autograd import forward_ad
 
 _LIB = None
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libdhellam_b200.so"
@@ -59,6 +60,15 @@ def use_native(t) -> bool:
 def use_library(t) -> bool:
     """True when an op on CUDA tensor ``t`` should run the PyTorch / vendor-library composition."""
     return t.is_cuda and _BACKEND == "library"
+
+
+def is_plain(t) -> bool:
+    """True for an ordinary tensor of the current device that nobody differentiates, traces or maps over: a kernel may
+    stand in for the PyTorch ops on it.  (Ops that have never been composed of PyTorch ops need no such question.)"""
+    return type(t) is torch.Tensor and t.is_cuda and t.device.index == torch.cuda.current_device() \
+        and not (t.requires_grad and torch.is_grad_enabled()) and forward_ad._current_level < 0 \
+        and torch._C._functorch.peek_interpreter_stack() is None and torch._C._len_torch_dispatch_stack() == 0 \
+        and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
 
 
 # Reproducible mode: every reduction whose order would depend on timing (norm weight gradients, the embedding

@@ -53,8 +53,8 @@ def _smoothing(label_smoothing: float, vocab: int) -> float:
 def ce_combine_stats(all_stats, label_smoothing: float = 0.0, vocab: int = 0):
     """``all_stats [R,T,4]`` -> ``(loss [T], lse [T])``; ``vocab`` = full vocabulary size (needed
     only with label smoothing)."""
-    if K.use_native(all_stats) and all_stats.dim() == 3 and all_stats.is_contiguous() and all_stats.dtype == torch.float32 \
-            and all_stats.data_ptr() % 16 == 0:
+    if K.use_native(all_stats) and K.is_plain(all_stats) and all_stats.dim() == 3 and all_stats.shape[0] > 0 and all_stats.shape[2] == 4 \
+            and all_stats.is_contiguous() and all_stats.dtype == torch.float32 and all_stats.data_ptr() % 16 == 0:
         R, T, _ = all_stats.shape
         loss = torch.empty(T, dtype=torch.float32, device=all_stats.device)
         lse = torch.empty_like(loss)

@@ -515,6 +515,28 @@ def test_ce_combine_against_the_composed_form(R, T, smoothing):
         assert rel(g, w) < 1e-6
 
 
+def test_ce_combine_leaves_to_the_composed_form_what_only_that_handles():
+    """Gradients (reverse and forward), a map over the statistics, no rank at all, no sums of logits, another stride: as on the CPU."""
+    from dhellam_b200.ops.loss import ce_combine_stats
+    stats, tangent = torch.rand(2, 5, 4) + 0.5, torch.randn(2, 5, 4)
+
+    def answers(dev):
+        s, t = stats.to(dev), tangent.to(dev)
+        leaf = s.clone().requires_grad_()
+        loss, lse = ce_combine_stats(leaf)
+        (loss.sum() + 2 * lse.sum()).backward()
+        yield leaf.grad
+        yield from torch.func.jvp(ce_combine_stats, (s,), (t,))[1]
+        yield from torch.func.vmap(ce_combine_stats)(torch.stack([s, s + 1]))
+        yield from ce_combine_stats(s[:, :, :3].contiguous())
+        yield from ce_combine_stats(s[:, ::2])
+        with pytest.raises((IndexError, RuntimeError)):
+            ce_combine_stats(s[:0])
+
+    for got, want in zip(answers(DEV), answers("cpu")):
+        assert rel(got, want) < 1e-6
+
+
 def test_bounded_wait_reports_timeout_without_hanging():
     """A flag that nobody sets: the device-side wait gives up after its (short) budget and
     the host reads the status word; the context stays usable."""
