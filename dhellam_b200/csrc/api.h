@@ -38,6 +38,8 @@ int dh_gemm_bf16(const void* a, int64_t lda, int a_mn_major, const void* b, int6
                  cudaStream_t stream);
 // Accepted and without effect: there is one dK/dV kernel.
 void dh_attn_set_bwd_mode(int mode);
+// Kernel launches that a packed forward over these sequences is cut into (tiles of 128 query rows); negative: a CUDA error code.
+int dh_attn_packed_launches(int nseq, const int* cu_q, const int* cu_k, int causal);
 // Kernel choice for dh_gemm_bf16: 0 = per problem (default; also DHELLAM_GEMM_MODE), 1 = single-CTA tiles
 // (128 x 256) only, 2 = CTA-pair tiles (256 x 256, tcgen05 cta_group::2) whenever M > 128.
 void dh_gemm_set_mode(int mode);

@@ -78,11 +78,12 @@ constexpr float LOG2E = 1.4426950408889634f;
 
 // Sequences and tiles of one packed launch (a kernel parameter: no device table, nothing to copy or keep).
 constexpr int MAX_SEQS = 128, MAX_TILES = 768;
+constexpr int TILE_BITS = 24;                // tiles of 128 rows of a sequence of up to 2^31 rows
 struct Packed {
   int q0[MAX_SEQS], k0[MAX_SEQS];            // first row in the packed tensors
   int nq[MAX_SEQS], nk[MAX_SEQS];            // rows
   int id[MAX_SEQS];                          // position in the batch (row of the statistics)
-  uint32_t tile[MAX_TILES];                  // sequence << 16 | tile
+  uint32_t tile[MAX_TILES];                  // sequence << TILE_BITS | tile
 };
 struct Dense {};                             // equal lengths: everything follows from the block index
 
@@ -111,8 +112,8 @@ __device__ __forceinline__ Work find_work(const Geometry& g, const Table& t, int
   if constexpr (sizeof(Table) > 1) {
     w.head = item % g.heads;
     const uint32_t e = t.tile[item / g.heads];
-    const int s = (int)(e >> 16);
-    w.tile = (int)(e & 0xffffu);
+    const int s = (int)(e >> TILE_BITS);
+    w.tile = (int)(e & ((1u << TILE_BITS) - 1));
     w.b = 0;
     w.sid = t.id[s];
     w.q0 = t.q0[s]; w.k0 = t.k0[s]; w.nq = t.nq[s]; w.nk = t.nk[s];
@@ -1135,8 +1136,7 @@ static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows
   std::vector<T> tiles;
   for (int s = 0; s < sq.n; ++s) {
     const int nq = sq.cu_q[s + 1] - sq.cu_q[s], nk = sq.cu_k[s + 1] - sq.cu_k[s];
-    const int n = (rows(nq, nk) + per - 1) / per;
-    if (n > 65536) { set_last_error("attention: a sequence of %d rows is longer than a packed batch supports", rows(nq, nk)); return cudaErrorInvalidValue; }
+    const int n = (int)(((long long)rows(nq, nk) + per - 1) / per);
     for (int t = 0; t < n; ++t) tiles.push_back({cost(nq, nk, t), s, t});
   }
   std::stable_sort(tiles.begin(), tiles.end(), [](const T& a, const T& b) { return a.cost > b.cost; });
@@ -1157,7 +1157,7 @@ static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows
       p.k0[ns] = sq.cu_k[t.seq]; p.nk[ns] = sq.cu_k[t.seq + 1] - sq.cu_k[t.seq];
       p.id[ns++] = t.seq;
     }
-    p.tile[nt++] = (uint32_t)slot[t.seq] << 16 | (uint32_t)t.tile;
+    p.tile[nt++] = (uint32_t)slot[t.seq] << TILE_BITS | (uint32_t)t.tile;
   }
   flush();
   return cudaSuccess;
@@ -1386,6 +1386,15 @@ int dh_attn_fwd_packed(const void* q, const void* k, const void* v, void* out, v
   e = cudaGetLastError();
   if (e != cudaSuccess) set_last_error("dh_attn_fwd_packed launch failed: %s", cudaGetErrorString(e));
   return (int)e;
+}
+
+int dh_attn_packed_launches(int nseq, const int* cu_q, const int* cu_k, int causal) {
+  const Sequences seqs = {nseq, cu_q, cu_k};
+  int launches = 0;
+  const cudaError_t e = for_packed_launches(seqs, BQ, [](int nq, int) { return nq; },
+                                            [&](int nq, int nk, int t) { return key_blocks(nq, nk, causal, t * BQ, BQ); },
+                                            [&](const Packed&, int) { ++launches; });
+  return e == cudaSuccess ? launches : -(int)e;
 }
 
 int64_t dh_attn_bwd_scratch_bytes(int B, int Hq, int Hk, int Sq, int Sk) {

@@ -56,3 +56,16 @@ def test_operands_that_the_kernels_would_misread_are_refused(which, how):
             attn_fwd_packed(o["q"], o["k"], o["v"], cu, cu, 30, True, None)
     with pytest.raises(AssertionError):
         attn_bwd_packed(o["dout"], o["q"], o["k"], o["v"], o["out"], o["lse"], o["dq"], o["dk"], o["dv"], cu, cu, True, None)
+
+
+def _launches(lengths, causal=1):
+    cu = [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    off, p_int = (c_int * len(cu))(*cu), ctypes.POINTER(c_int)
+    return K.proto("dh_attn_packed_launches", [c_int, p_int, p_int, c_int])(len(lengths), off, off, causal)
+
+
+def test_a_long_sequence_is_cut_into_launches():
+    """A tile's index fits its field of the launch's table whatever the length: 2^24 rows are 131072 tiles, 768 to a launch."""
+    assert _launches([2 ** 24, 100]) == 171
