@@ -59,6 +59,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -1131,7 +1132,7 @@ struct Sequences {
   const int* cu_k;
 };
 template <class Rows, class Cost, class F>
-static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows, Cost&& cost, F&& launch) {
+static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows, Cost&& cost, F&& launch) try {
   struct T { long long cost; int seq, tile; };
   std::vector<T> tiles;
   for (int s = 0; s < sq.n; ++s) {
@@ -1161,6 +1162,9 @@ static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows
   }
   flush();
   return cudaSuccess;
+} catch (const std::bad_alloc&) {          // no exception may leave a C entry point
+  set_last_error("attention: no host memory for the list of tiles");
+  return cudaErrorMemoryAllocation;
 }
 static bool offsets_ok(const char* who, const Sequences& s, int Tq, int Tk, int max_q) {
   for (int i = 0; i < s.n; ++i) {

@@ -1,5 +1,8 @@
 """What the packed attention entry points accept and refuse before they launch anything (CPU)."""
 import ctypes
+import os
+import subprocess
+import sys
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import pytest
@@ -69,3 +72,18 @@ def _launches(lengths, causal=1):
 def test_a_long_sequence_is_cut_into_launches():
     """A tile's index fits its field of the launch's table whatever the length: 2^24 rows are 131072 tiles, 768 to a launch."""
     assert _launches([2 ** 24, 100]) == 171
+
+
+def test_a_failed_host_allocation_is_an_error_code():
+    """The list of tiles of 2^30 rows does not fit what the process may still allocate: the C entry point answers, it does not abort."""
+    code = """
+import resource
+from test_attention_packed_limits import _launches
+assert _launches([1000]) == 1
+used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (used + (64 << 20), -1))
+assert _launches([2 ** 30]) == -2                # out of memory, as a CUDA error code
+"""
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join(sys.path))
+    run = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True)
+    assert run.returncode == 0, run.stderr
