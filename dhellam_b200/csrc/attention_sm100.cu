@@ -1124,43 +1124,45 @@ static void launch_in_waves(long long items, int sm_budget, F&& launch) {
   for (long long x0 = 0; x0 < items; x0 += wave) launch((unsigned)std::min(wave, items - x0), (int)x0);
 }
 
-// Tiles of a packed batch in descending order of work, cut into launches that fit one kernel parameter.
-// work(nq, nk, tile) = key (query) blocks of that tile; rows(nq, nk) = what the tiles cover, `per` rows each.
+// Tiles of a packed batch in descending order of work, cut into launches that fit one kernel parameter: MAX_TILES tiles of at most
+// MAX_SEQS sequences.  More sequences are divided by length first (the longest MAX_SEQS, the next, ...): sorted as one, the equal
+// tiles of all sequences would stand side by side and every MAX_SEQS of them fill a table (300 causal sequences of 1024 rows: 19
+// launches, like this 5).
+// rows(nq, nk) = what the tiles cover, `per` rows each; cost(nq, nk, tile) = key (query) blocks of that tile.
 struct Sequences {
   int n;
   const int* cu_q;
   const int* cu_k;
+  int nq(int s) const { return cu_q[s + 1] - cu_q[s]; }
+  int nk(int s) const { return cu_k[s + 1] - cu_k[s]; }
 };
 template <class Rows, class Cost, class F>
 static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows, Cost&& cost, F&& launch) try {
-  struct T { long long cost; int seq, tile; };
+  struct T { long long cost; int slot, tile; };
+  std::vector<int> order(sq.n);
+  for (int s = 0; s < sq.n; ++s) order[s] = s;
+  if (sq.n > MAX_SEQS) {
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rows(sq.nq(a), sq.nk(a)) > rows(sq.nq(b), sq.nk(b)); });
+  }
   std::vector<T> tiles;
-  for (int s = 0; s < sq.n; ++s) {
-    const int nq = sq.cu_q[s + 1] - sq.cu_q[s], nk = sq.cu_k[s + 1] - sq.cu_k[s];
-    const int n = (int)(((long long)rows(nq, nk) + per - 1) / per);
-    for (int t = 0; t < n; ++t) tiles.push_back({cost(nq, nk, t), s, t});
-  }
-  std::stable_sort(tiles.begin(), tiles.end(), [](const T& a, const T& b) { return a.cost > b.cost; });
-  std::vector<int> slot(sq.n, -1);
-  Packed p;
-  int ns = 0, nt = 0;
-  auto flush = [&]() {
-    if (nt == 0) return;
-    launch(p, nt);
-    for (int i = 0; i < ns; ++i) slot[p.id[i]] = -1;
-    ns = nt = 0;
-  };
-  for (const T& t : tiles) {
-    if (nt == MAX_TILES || (slot[t.seq] < 0 && ns == MAX_SEQS)) flush();
-    if (slot[t.seq] < 0) {
-      slot[t.seq] = ns;
-      p.q0[ns] = sq.cu_q[t.seq]; p.nq[ns] = sq.cu_q[t.seq + 1] - sq.cu_q[t.seq];
-      p.k0[ns] = sq.cu_k[t.seq]; p.nk[ns] = sq.cu_k[t.seq + 1] - sq.cu_k[t.seq];
-      p.id[ns++] = t.seq;
+  for (int first = 0; first < sq.n; first += MAX_SEQS) {
+    Packed p;
+    tiles.clear();
+    for (int i = 0; i < MAX_SEQS && first + i < sq.n; ++i) {
+      const int s = order[first + i], nq = sq.nq(s), nk = sq.nk(s);
+      p.q0[i] = sq.cu_q[s]; p.nq[i] = nq;
+      p.k0[i] = sq.cu_k[s]; p.nk[i] = nk;
+      p.id[i] = s;
+      const int n = (int)(((long long)rows(nq, nk) + per - 1) / per);
+      for (int t = 0; t < n; ++t) tiles.push_back({cost(nq, nk, t), i, t});
     }
-    p.tile[nt++] = (uint32_t)slot[t.seq] << TILE_BITS | (uint32_t)t.tile;
+    std::stable_sort(tiles.begin(), tiles.end(), [](const T& a, const T& b) { return a.cost > b.cost; });
+    for (size_t t0 = 0; t0 < tiles.size(); t0 += MAX_TILES) {
+      const int nt = (int)std::min(tiles.size() - t0, (size_t)MAX_TILES);
+      for (int t = 0; t < nt; ++t) p.tile[t] = (uint32_t)tiles[t0 + t].slot << TILE_BITS | (uint32_t)tiles[t0 + t].tile;
+      launch(p, nt);
+    }
   }
-  flush();
   return cudaSuccess;
 } catch (const std::bad_alloc&) {          // no exception may leave a C entry point
   set_last_error("attention: no host memory for the list of tiles");
@@ -1168,7 +1170,7 @@ static cudaError_t for_packed_launches(const Sequences& sq, int per, Rows&& rows
 }
 static bool offsets_ok(const char* who, const Sequences& s, int Tq, int Tk, int max_q) {
   for (int i = 0; i < s.n; ++i) {
-    const int nq = s.cu_q[i + 1] - s.cu_q[i], nk = s.cu_k[i + 1] - s.cu_k[i];
+    const int nq = s.nq(i), nk = s.nk(i);
     if (s.cu_q[i] < 0 || s.cu_k[i] < 0 || nq < 0 || nk < 0 || nq > max_q || s.cu_q[i + 1] > Tq || s.cu_k[i + 1] > Tk) {
       set_last_error("%s: sequence %d (queries %d..%d, keys %d..%d) does not fit the packed tensors or the longest length %d", who, i,
                      s.cu_q[i], s.cu_q[i + 1], s.cu_k[i], s.cu_k[i + 1], max_q);

@@ -74,6 +74,14 @@ def test_a_long_sequence_is_cut_into_launches():
     assert _launches([2 ** 24, 100]) == 171
 
 
+@pytest.mark.parametrize("lengths,most", [([1024] * 300, 5), ([128] * 1024, 8), ([64] * 129, 2), ([0] * 500 + [4096] * 24, 5),
+                                          ([17 + 31 * (i % 97) for i in range(640)], 13), ([8192] * 64, 6)])
+def test_many_sequences_take_about_as_few_launches_as_their_tables_allow(lengths, most):
+    """At most 768 tiles of 128 sequences to a launch; a batch of more sequences is divided by length before its tiles are sorted."""
+    tiles = sum((n + 127) // 128 for n in lengths)
+    assert max(-(-tiles // 768), -(-sum(n > 0 for n in lengths) // 128)) <= _launches(lengths) <= most
+
+
 def test_a_failed_host_allocation_is_an_error_code():
     """The list of tiles of 2^30 rows does not fit what the process may still allocate: the C entry point answers, it does not abort."""
     code = """
