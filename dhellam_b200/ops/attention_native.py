@@ -77,6 +77,8 @@ def attn_fwd_packed(q, k, v, cq, ck, max_q, causal, scale, sm_budget=0, stream=N
     shape = (b, Hq, max_q)
     lse = torch.empty(shape, dtype=torch.float32, device=q.device) if whole else \
         torch.full(shape, float("-inf"), dtype=torch.float32, device=q.device)
+    if Tk == 0:                                  # no key anywhere, nothing to launch
+        return out.zero_(), lse.fill_(float("-inf"))
     fn = K.proto("dh_attn_fwd_packed", [c_void_p] * 5 + [ctypes.POINTER(c_int64), c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int),
                                                          c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
     K.check(fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), (c_int64 * 8)(*(s for p in strides for s in p)), b,
@@ -93,6 +95,10 @@ def attn_bwd_packed(dout, q, k, v, out, lse, dq, dk, dv, cq, ck, causal, scale, 
         strides += (row, row, head)
     Tq, Tk = min(t.shape[0] for t in (q, dout, out, dq)), min(t.shape[0] for t in (k, v, dk, dv))
     assert cq[-1] <= Tq and ck[-1] <= Tk and lse.dtype == torch.float32 and lse.get_device() == device
+    if Tq == 0 or Tk == 0:
+        for t in (dq, dk, dv):
+            t.zero_()
+        return
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
     lse = lse.contiguous()
     b = len(cq) - 1

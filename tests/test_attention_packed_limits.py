@@ -61,6 +61,20 @@ def test_operands_that_the_kernels_would_misread_are_refused(which, how):
         attn_bwd_packed(o["dout"], o["q"], o["k"], o["v"], o["out"], o["lse"], o["dq"], o["dk"], o["dv"], cu, cu, True, None)
 
 
+@pytest.mark.parametrize("tq,tk", [(50, 0), (0, 50), (0, 0)])
+def test_batches_without_any_key_or_query_give_zeros(tq, tk):
+    """As the empty sequences of a batch that has others: no probability, no gradient."""
+    from dhellam_b200.ops.attention_native import attn_bwd_packed, attn_fwd_packed
+    o = {n: torch.full_like(t, float("nan")) for n, t in _operands(tq, tk).items()}
+    cq, ck = [0, tq * 2 // 5, tq], [0, tk * 2 // 5, tk]
+    if tk == 0:
+        for max_q in (30, 40):
+            out, lse = attn_fwd_packed(o["q"], o["k"], o["v"], cq, ck, max_q, True, None)
+            assert out.shape == o["q"].shape and not out.any() and lse.shape == (2, 2, max_q) and (lse == float("-inf")).all()
+    attn_bwd_packed(o["dout"], o["q"], o["k"], o["v"], o["out"], o["lse"], o["dq"], o["dk"], o["dv"], cq, ck, True, None)
+    assert not any(o[n].any() for n in ("dq", "dk", "dv"))
+
+
 def _launches(lengths, causal=1):
     cu = [0]
     for n in lengths:
