@@ -48,6 +48,8 @@ void dh_gemm_set_mode(int mode);
 void dh_gemm_set_splitk(int n);
 // Small-output kernel (128 x 128 tiles, K divided over a cluster of up to 8 CTAs): -1 = by problem, 0 = never, n = n CTAs.
 void dh_gemm_set_cluster_k(int n);
+// What that choice is for a problem on `sms` SMs: CTAs per tile, 0 = one of the other kernels.
+int dh_gemm_cluster_k(int M, int N, int K, int out_f32, int sms);
 // dh_gemm_bf16 with the tensor-parallel collective hooks of the CTA-pair kernel (see gemm_sm100.cu).
 int dh_gemm_bf16_sync(const void* a, int64_t lda, int a_mn_major, const void* b, int64_t ldb, int b_mn_major, void* d, int64_t ldd,
                       int d_fp32, int accumulate, int M, int N, int K, int sm_budget, const void* wait_count, unsigned wait_target,

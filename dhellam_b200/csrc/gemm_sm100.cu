@@ -1084,12 +1084,19 @@ static int choose_split_k(int tiles, int pairs, int num_kb) {
 // Forced by dh_gemm_set_cluster_k: -1 = this rule, 0 = never, n = n CTAs (as far as K allows).
 static int g_cluster_k = -1;
 
-// The rule, from a sweep of 8 to 2048 rows against weights of 512 x 512 to 28672 x 4096 (times with 10 us of launch and event
-// in them, pair kernel -> this one): up to a quarter of the SMs' worth of tiles, 4 CTAs per tile (128 x 4096 x 4096 36 -> 19 us,
-// 512 x 1024 x 1024 15.4 -> 12.3 us); up to half, 2, or 4 where K is long (200 x 4096 x 14336 78 -> 47 us, x 4096 31 -> 23 us); up to one
-// tile per SM, 2 where K is long enough to pay for the reduction (300 x 4096 x 14336 80 -> 66 us, 300 x 6144 x 4096 34 -> 32 us; but
-// 2048 x 1024 x 1024 15 -> 18 us). With more tiles the pair kernel's larger tiles read less through L2 and win (512 x 6144 x 4096 35
-// against 45 us), as it does for fp32 outputs of more than one row of tiles (1024 x 1024 x 1024 17 against 18 us and up).
+// The rule, from sweeps of 1 to 2048 rows against weights of 512 x 512 to 28672 x 4096, all three layouts (us of back-to-back
+// launches over operands that exceed L2, other kernel -> this one with that many CTAs per tile):
+//   up to 33 tiles, 4: 33 clusters of four find room at once on 148 SMs (34 do not: 64 rows, 34 tiles, 1024 deep 12.4 -> 16.5 with 4);
+//     128 rows, 28 tiles, 4096 deep 32.9 -> 14.5, 8 rows, 18 tiles, 512 deep 8.3 -> 8.1;
+//   up to half the SMs, 2 from 1024 deep on (256 rows, 38 tiles, 2048 deep 16.6 -> 14.3; 74 tiles, 6144 deep 36.4 -> 22.6), or 4 where K is
+//     long and two CTAs per SM hold the clusters (64 rows, 64 tiles, 12288 deep 80 -> 41; 72 tiles 64 with 4, 45 with 2);
+//   up to one tile per SM, 2 where K is long enough to pay for the reduction.  That depends on the rows, because below 128 of them
+//     the single-CTA kernel is the other one and streams the weight the better the fewer there are: from 4096 deep on (300 x 111 tiles
+//     27.2 -> 25.3), up to 128 rows from 2048 (128 x 96 tiles 21.2 -> 18.5; 64 x 128 tiles 20.6 -> 22.6), up to 96 from 3072 (64 x 112
+//     28.0 -> 25.2; 16 x 96 26.7 -> 37.2), below 24 from 4096 (16 x 96 32.8 -> 25.3; 8 x 75 31.2 -> 39.3), below 16 from 8192
+//     (8 x 96 55.1 -> 41.3).  fp32 outputs likewise but not below 64 rows (8 x 147 tiles, 8192 deep 70 -> 80).
+// With more tiles the pair kernel's larger tiles read less through L2 and win (512 x 6144 x 4096 35 against 45 us), as it does for
+// fp32 outputs of more than one row of tiles (1024 x 1024 x 1024 17 against 18 us and up).
 static int choose_cluster_k(int M, int N, int num_kb, int out_f32, int sms) {
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + small::TILE_N - 1) / small::TILE_N);
   if (tiles * small::MAX_CLUSTER > (1ll << 30)) return 0;
@@ -1099,9 +1106,12 @@ static int choose_cluster_k(int M, int N, int num_kb, int out_f32, int sms) {
     return c;
   }
   if (tiles > sms || (out_f32 && M > BM)) return 0;
-  if (tiles * 4 <= sms) return num_kb >= 8 ? 4 : 0;
-  if (tiles * 2 <= sms) return num_kb >= 192 ? 4 : (num_kb >= 16 ? 2 : 0);
-  return num_kb >= (M <= BM ? 32 : 64) ? 2 : 0;
+  const long long fours = sms * 33ll / 148;                     // clusters of four that are resident at one CTA per SM
+  if (tiles <= fours) return num_kb >= 8 ? 4 : 0;
+  if (tiles * 2 <= sms) return num_kb >= 192 && tiles <= 2 * fours ? 4 : (num_kb >= 16 ? 2 : 0);
+  if (out_f32 && M < 64) return 0;
+  const int from = M > BM ? 64 : (M > 96 ? 32 : (M >= 24 ? 48 : (M >= 16 ? 64 : 128)));
+  return num_kb >= from ? 2 : 0;
 }
 
 struct SyncArgs {
@@ -1275,6 +1285,10 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
 extern "C" void dh_gemm_set_splitk(int n) { dh::gemm::g_splitk_override = n; }
 
 // Small-output kernel (128 x 128 tiles, K over a cluster): -1 = by problem (default), 0 = never, n = n CTAs per tile.
+// That rule (or the forced number) for a problem on `sms` SMs.
+extern "C" int dh_gemm_cluster_k(int M, int N, int K, int out_f32, int sms) {
+  return dh::gemm::choose_cluster_k(M, N, (K + dh::gemm::BK - 1) / dh::gemm::BK, out_f32, sms);
+}
 extern "C" void dh_gemm_set_cluster_k(int n) { dh::gemm::g_cluster_k = n; }
 
 extern "C" int dh_gemm_bf16(const void* a, int64_t lda, int a_mn_major, const void* b, int64_t ldb, int b_mn_major, void* d,
