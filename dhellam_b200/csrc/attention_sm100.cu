@@ -7,7 +7,8 @@
 // units, so the kernels are built to keep both busy at once:
 //
 // Forward, one CTA per two tiles of 128 query rows that share their keys (two query heads of a
-// KV group; for groups of odd size two neighbouring row tiles of one head):
+// KV group; for groups of odd size two neighbouring row tiles of one head; one tile where that
+// leaves no SM with two, fwd_mode):
 //   warp 0      TMA producer: Q tiles once, then K_j / V_j through one 5-slot ring
 //   warp 1      MMA issuer:   S_t = Q_t K_j^T, O_t += P_t V_j (t = 0, 1) with P read from TMEM
 //   warps 4-7, 8-11  softmax of tile 0 / 1: one thread per row, no exchange between threads; P_t
@@ -201,8 +202,9 @@ struct FwdArgs {
   __nv_bfloat16* out;
   float* lse;
   long long o_s, o_b, o_h;                   // output strides (elements)
-  int head_pair;                             // 1: a CTA's two tiles are query heads 2h, 2h+1; 0: row tiles 2i, 2i+1 of one head
+  int mode;                                  // what a CTA's two tiles are:
 };
+enum { ROW_PAIR, HEAD_PAIR, SINGLE };        // row tiles 2i, 2i+1 of one head; query heads 2h, 2h+1; one tile only, the second is empty
 
 // POSITIVE: the scale is; a form of its own for the others, whose masked keys need more than a score of -inf (as one
 // kernel 3 % slower for everybody).
@@ -219,13 +221,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const Work w = find_work(g, table, g.x0 + (int)blockIdx.x);
   const int off = w.nk - w.nq;                     // key j visible to query i iff j <= i + off
-  const int hq_[2] = {a.head_pair ? 2 * w.head : w.head, a.head_pair ? 2 * w.head + 1 : w.head};
+  const int hq_[2] = {a.mode == HEAD_PAIR ? 2 * w.head : w.head, a.mode == HEAD_PAIR ? 2 * w.head + 1 : w.head};
   const int hk = hq_[0] / (g.Hq / g.Hk);
   // dense tiles are counted from the end: the latest queries see most keys
-  const int per_cta = a.head_pair ? BQ : 2 * BQ;
+  const int per_cta = a.mode == ROW_PAIR ? 2 * BQ : BQ;
   const int last = (w.nq + per_cta - 1) / per_cta - 1;
   const int tile = sizeof(Table) > 1 ? w.tile : last - w.tile;
-  const int qb_[2] = {a.head_pair ? tile : 2 * tile, a.head_pair ? tile : 2 * tile + 1};
+  const int qb_[2] = {a.mode == ROW_PAIR ? 2 * tile : tile,
+                      a.mode == ROW_PAIR ? 2 * tile + 1 : (a.mode == HEAD_PAIR ? tile : (w.nq + BQ - 1) / BQ)};
   int nblk_[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
@@ -1204,9 +1207,37 @@ static void run_fwd(const FwdMaps& m, Geometry& g, const FwdArgs& a, const Table
   });
 }
 
-// Two query heads of a KV group per CTA where groups are even: both tiles then see the same keys whatever the mask, and
+static long long packed_tiles(int nseq, const int* cu) {        // of 128 rows, in all sequences
+  long long n = 0;
+  for (int s = 0; s < nseq; ++s) n += (cu[s + 1] - cu[s] + BQ - 1) / BQ;
+  return n;
+}
+
+// What a CTA of the forward takes.  One tile where every tile finds an SM of its own: it then does not wait for another's products and
+// exponentials (1000 positions, 8 heads on 1, all keys: 24.7 -> 20.6 us, 2048: 41.5 -> 34.4).  Also where the longest tile alone takes as
+// long as all of them spread over the SMs, that is under causal masks (up to twice as many tiles as SMs were measured; 4096
+// positions, 8 heads on 1: 71 -> 60 us), unless tiles are so short that a second round of CTAs costs more (384 positions: 14.4 -> 16.5).
+// Else two query heads of a KV group where groups are even: both tiles then see the same keys whatever the mask, and
 // a sequence of up to 128 rows fills the CTA.  Odd groups (one query head per KV head) take two row tiles instead.
-static int fwd_head_pair(int Hq, int Hk) { return (Hq / Hk) % 2 == 0; }
+static int fwd_mode(const Sequences& sq, int B, int Hq, int Hk, int causal, int sm_budget) {
+  const int sms = dh_sm_count();
+  const bool budgeted = sm_budget > 0 && sm_budget < sms;
+  const long long room = budgeted ? sm_budget : sms, per_tile = (long long)B * Hq;
+  const long long tiles = packed_tiles(sq.n, sq.cu_q) * per_tile;
+  if (tiles <= room) return SINGLE;
+  if (!budgeted && tiles <= 2 * room) {
+    long long work = 0, longest = 0;
+    for (int s = 0; s < sq.n; ++s) {
+      for (int first = 0; first < sq.nq(s); first += BQ) {
+        const long long n = key_blocks(sq.nq(s), sq.nk(s), causal, first, BQ);
+        work += n;
+        longest = std::max(longest, n);
+      }
+    }
+    if (longest >= 8 && work * per_tile <= room * longest) return SINGLE;
+  }
+  return (Hq / Hk) % 2 == 0 ? HEAD_PAIR : ROW_PAIR;
+}
 
 // Number of CTAs that share the query heads of one KV head in the dK/dV kernel: 1 while
 // KV blocks x batch x KV heads already give every SM a few CTAs, else the smallest power of
@@ -1223,11 +1254,6 @@ static int bwd_head_split(long long kv_tiles, int Hq, int Hk) {
   int hs = 1;
   while (hs < group && group % (hs * 2) == 0 && ctas * hs < 4LL * dh_sm_count()) hs *= 2;
   return hs;
-}
-static long long packed_kv_tiles(int nseq, const int* cu_k) {
-  long long n = 0;
-  for (int s = 0; s < nseq; ++s) n += (cu_k[s + 1] - cu_k[s] + BKV - 1) / BKV;
-  return n;
 }
 // Scratch of the backward: delta [B*Hq*Tq] fp32 (row dot products of dO and O), rounded up to 256 bytes, then, when
 // the dK/dV kernel splits heads, the fp32 partials [2][hs][Tk][B][Hk][128].
@@ -1356,9 +1382,10 @@ int dh_attn_fwd(const void* q, const void* k, const void* v, void* out, void* ls
   FwdArgs a;
   a.out = (__nv_bfloat16*)out; a.lse = (float*)lse;
   a.o_h = D; a.o_b = (long long)Hq * D; a.o_s = (long long)B * Hq * D;
-  a.head_pair = fwd_head_pair(Hq, Hk);
-  const int per = a.head_pair ? BQ : 2 * BQ;
-  g.heads = a.head_pair ? Hq / 2 : Hq;
+  const int cu_q[2] = {0, Sq}, cu_k[2] = {0, Sk};
+  a.mode = fwd_mode({1, cu_q, cu_k}, B, Hq, Hk, causal, sm_budget);
+  const int per = a.mode == ROW_PAIR ? 2 * BQ : BQ;
+  g.heads = a.mode == HEAD_PAIR ? Hq / 2 : Hq;
   run_fwd(m, g, a, Dense{}, (long long)((Sq + per - 1) / per) * g.heads * B, sm_budget, stream);
   e = cudaGetLastError();
   if (e != cudaSuccess) set_last_error("dh_attn_fwd launch failed: %s", cudaGetErrorString(e));
@@ -1382,9 +1409,9 @@ int dh_attn_fwd_packed(const void* q, const void* k, const void* v, void* out, v
   FwdArgs a;
   a.out = (__nv_bfloat16*)out; a.lse = (float*)lse;
   a.o_s = strides[6]; a.o_h = strides[7]; a.o_b = 0;
-  a.head_pair = fwd_head_pair(Hq, Hk);
-  const int per = a.head_pair ? BQ : 2 * BQ;
-  g.heads = a.head_pair ? Hq / 2 : Hq;
+  a.mode = fwd_mode(seqs, 1, Hq, Hk, causal, sm_budget);
+  const int per = a.mode == ROW_PAIR ? 2 * BQ : BQ;
+  g.heads = a.mode == HEAD_PAIR ? Hq / 2 : Hq;
   e = for_packed_launches(seqs, per, [](int nq, int) { return nq; },
                           [&](int nq, int nk, int t) { return key_blocks(nq, nk, causal, t * per, per); },
                           [&](const Packed& p, int n) { run_fwd(m, g, a, p, (long long)n * g.heads, sm_budget, stream); });
@@ -1409,7 +1436,7 @@ int64_t dh_attn_bwd_scratch_bytes(int B, int Hq, int Hk, int Sq, int Sk) {
 }
 
 int64_t dh_attn_bwd_packed_scratch_bytes(int nseq, const int* cu_k, int Hq, int Hk, int Tq, int Tk) {
-  const int hs = Hk > 0 && Hq % Hk == 0 ? bwd_head_split(packed_kv_tiles(nseq, cu_k), Hq, Hk) : 1;
+  const int hs = Hk > 0 && Hq % Hk == 0 ? bwd_head_split(packed_tiles(nseq, cu_k), Hq, Hk) : 1;
   return scratch_bytes(1, Hq, Hk, Tq, Tk, hs);
 }
 
@@ -1455,7 +1482,7 @@ int dh_attn_bwd_packed(const void* dout, const void* q, const void* k, const voi
   if (!m.q || !m.k || !m.v || !m.dout) return (int)cudaErrorInvalidValue;
   cudaError_t e = opt_in_bwd<Packed>();
   if (e != cudaSuccess) return (int)e;
-  const int hs = bwd_head_split(packed_kv_tiles(nseq, cu_k), Hq, Hk);
+  const int hs = bwd_head_split(packed_tiles(nseq, cu_k), Hq, Hk);
   return bwd_common(dout, out, lse, dq, dk, dv, scratch, strides, m, geometry(1, Hq, Hk, 0, 0, Tq, Tk, lse_rows, causal, scale), hs, &seqs,
                     sm_budget, stream);
 }

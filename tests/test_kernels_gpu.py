@@ -447,6 +447,27 @@ def test_varlen_api_with_equal_lengths_uses_strided_views_of_the_packed_tensors(
         assert rel(sb(a), r) < 1e-3
 
 
+@pytest.mark.parametrize("Sq,Sk,Hq,Hk,causal", [(300, 300, 4, 2, True), (300, 300, 3, 1, True), (129, 400, 2, 2, False),
+                                                (400, 129, 6, 2, True), (128, 128, 2, 1, True)])
+def test_attention_forward_is_the_same_however_tiles_share_ctas(Sq, Sk, Hq, Hk, causal):
+    """One tile per CTA (as these sizes run by themselves) and two heads or two row tiles per CTA (with an SM budget that has no room
+    for a CTA each), dense and packed: bitwise the same."""
+    from dhellam_b200.ops.attention import attn_fwd, pymha_varlen_fwd
+    q, k, v = bf(Sq, 2, Hq, 128), bf(Sk, 2, Hk, 128), bf(Sk, 2, Hk, 128)
+    o, lse = attn_fwd(q, k, v, causal)
+    for budget in (1, 5):
+        o2, lse2 = attn_fwd(q, k, v, causal, sm_budget=budget)
+        assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    pack = lambda t, last: torch.cat([t[:, 0], t[:last, 1]])      # the second sequence is 37 rows shorter
+    cq, ck = [0, Sq, 2 * Sq - 37], [0, Sk, 2 * Sk - 37]
+    packed = pack(q, Sq - 37), pack(k, Sk - 37), pack(v, Sk - 37)
+    out, lse3 = pymha_varlen_fwd(*packed, cq, ck, Sq, Sk, is_causal=causal)
+    assert torch.equal(out[:Sq], o[:, 0]) and torch.equal(lse3[0], lse[0])
+    for budget in (1, 5):
+        out2, lse4 = pymha_varlen_fwd(*packed, cq, ck, Sq, Sk, is_causal=causal, math_sm_count=budget)
+        assert torch.equal(out, out2) and torch.equal(lse3, lse4)
+
+
 @pytest.mark.parametrize("n,m", [(2, 2), (17, 5), (2000, 2096), (2000, 2097)])
 def test_offsets_on_the_device_are_read_as_they_are(n, m):
     """Up to the capacity of the pinned buffer in one read, beyond it one by one; int64 and strided tensors too."""
