@@ -138,6 +138,24 @@ def test_gemm_cluster_k(M, N, Kd, cluster):
     assert rel(g, 1 + dyt.double().t() @ xt.double()) < 1e-5
 
 
+@pytest.mark.parametrize("M,N,Kd", [(128, 4224, 512), (64, 4352, 1024), (8, 4608, 512), (64, 8192, 12288), (129, 6144, 4096),
+                                    (129, 6144, 4032), (16, 12288, 4096), (64, 12288, 4096), (300, 6528, 4096)])
+def test_gemm_by_the_rule(M, N, Kd):
+    """No kernel forced: problems on both sides of the lines between the kernels, bf16 and fp32 outputs, stored and accumulated.
+    bf16 rounding, and fp32 sums of Kd products in another order."""
+    from dhellam_b200.ops.gemm import gemm_nn, gemm_nt, gemm_tn_acc
+    x, w = bf(M, Kd), bf(N, Kd, scale=0.05)
+    ref = x.double() @ w.double().t()
+    assert rel(gemm_nt(x, w), ref) < 5e-3 and rel(gemm_nt(x, w, out_dtype=torch.float32), ref) < 1e-5
+    assert rel(gemm_nn(x, w.t().contiguous()), ref) < 5e-3
+    rows = 8 * ((M + 7) // 8)                              # fp32 rows of the accumulated output: M of them are looked at
+    dy = torch.zeros(Kd, rows, dtype=torch.bfloat16, device=DEV)
+    dy[:, :M] = x.t()
+    g = torch.ones(rows, N, device=DEV)
+    gemm_tn_acc(dy, w.t().contiguous(), g)
+    assert rel(g[:M] - 1, ref) < 1e-5 + 1e-7 * math.sqrt(M * N) / ref.norm().item()
+
+
 @pytest.mark.parametrize("rows,h", [(64, 256), (300, 4096), (257, 8192), (33, 1024)])
 def test_rmsnorm(rows, h, reduction_mode):
     from dhellam_b200.ops.norm import rmsnorm_bwd, rmsnorm_fwd
@@ -251,25 +269,17 @@ def test_router_topk():
     assert rel(gates.cpu()[same], gr[same]) < 1e-3
 
 
-@pytest.fixture(params=[0, 1], ids=["tile128", "pipelined64"])
-def attn_bwd_mode(request):
-    """Both dK/dV kernels: the default and the pipelined transposed-score form."""
-    from dhellam_b200.ops.attention import set_attn_bwd_mode
-    set_attn_bwd_mode(request.param)
-    yield request.param
-    set_attn_bwd_mode(0)
-
-
 @pytest.mark.parametrize("rows,h", [(1, 8), (3, 264), (700, 1000), (5, 8192), (4, 8200), (2, 16384)])
 @pytest.mark.parametrize("kind", ["rms", "layer"])
-def test_norm_backward_row_lengths(rows, h, kind):
+@pytest.mark.parametrize("residual", [False, True], ids=["plain", "residual"])
+def test_norm_backward_row_lengths(rows, h, kind, residual):
     """One vector per thread (up to 8192 elements, lanes to spare at 264 and 1000), several beyond; more rows than CTAs; with and
     without a residual, and a gradient buffer that is only 4-byte aligned.  bf16 results: 1e-2; fp32 sums: 1e-3."""
     from dhellam_b200.ops.norm import layernorm_bwd, layernorm_fwd, rmsnorm_bwd, rmsnorm_fwd
-    x, w, b, dy, res = bf(rows, h), bf(h), bf(h), bf(rows, h), bf(rows, h)
+    x, w, b, dy, res = bf(rows, h), bf(h), bf(h), bf(rows, h), bf(rows, h) if residual else None
     grads = torch.zeros(2, h + 1, device=DEV)
     dw, db, dwr, dbr = grads[0, 1:], grads[1, 1:], torch.zeros(h), torch.zeros(h)
-    cpu = lambda *t: [a.cpu().float() for a in t]
+    cpu = lambda *t: [a if a is None else a.cpu().float() for a in t]
     xc, wc, bc, dyc, rc = cpu(x, w, b, dy, res)
     if kind == "rms":
         _, rstd = rmsnorm_fwd(x, w)
@@ -277,15 +287,15 @@ def test_norm_backward_row_lengths(rows, h, kind):
         dxr, _ = rmsnorm_bwd(dyc, xc, wc, rstd.cpu(), weight_main_grad=dwr, residual_grad=rc)
     else:
         _, mu, rstd = layernorm_fwd(x, w, b)
-        dx, _, _ = layernorm_bwd(dy, x, w, mu, rstd, weight_main_grad=dw, bias_main_grad=db)
-        dxr, _, _ = layernorm_bwd(dyc, xc, wc, mu.cpu(), rstd.cpu(), weight_main_grad=dwr, bias_main_grad=dbr)
+        dx, _, _ = layernorm_bwd(dy, x, w, mu, rstd, weight_main_grad=dw, bias_main_grad=db, residual_grad=res)
+        dxr, _, _ = layernorm_bwd(dyc, xc, wc, mu.cpu(), rstd.cpu(), weight_main_grad=dwr, bias_main_grad=dbr, residual_grad=rc)
         assert rel(db, dbr) < 1e-3
     assert rel(dx, dxr) < 1e-2 and rel(dw, dwr) < 1e-3
 
 
 @pytest.mark.parametrize("Sq,Sk,B,Hq,Hk,causal", [(128, 128, 1, 1, 1, True), (256, 256, 2, 4, 2, True), (384, 384, 1, 2, 1, False),
                                                      (200, 200, 2, 2, 2, True), (128, 256, 1, 2, 1, False), (256, 128, 1, 2, 2, False)])
-def test_attention_forward_backward(Sq, Sk, B, Hq, Hk, causal, attn_bwd_mode):
+def test_attention_forward_backward(Sq, Sk, B, Hq, Hk, causal):
     from dhellam_b200.ops.attention import attn_bwd, attn_fwd
     d = 128
     # strided views into packed buffers, as the engine uses them
@@ -410,9 +420,8 @@ def test_attention_with_a_scale_that_is_not_positive(scale):
 
 @pytest.mark.parametrize("budget", [1, 5, 24, 100])
 def test_attention_sm_budget_gives_identical_results(budget):
-    """With an SM budget the attention kernels run as consecutive launches of at most that many CTAs
-    (tile columns split when one head alone has more tiles than the budget, else whole (head, batch)
-    pairs per launch); every tile computes exactly what it computes without a budget."""
+    """With an SM budget the work items of the attention kernels are cut into consecutive launches of at most that many CTAs;
+    every tile computes exactly what it computes without a budget."""
     from dhellam_b200.ops.attention import attn_bwd, attn_fwd
     Sq, B, Hq, Hk, d = 1024, 2, 4, 2, 128
     qkv = bf(Sq, B, Hq + 2 * Hk, d)
@@ -429,9 +438,9 @@ def test_attention_sm_budget_gives_identical_results(budget):
         assert torch.equal(a, b)
 
 
-def test_varlen_api_with_equal_lengths_uses_strided_views_of_the_packed_tensors():
-    """``pymha_varlen_fwd / bwd`` on a packed batch of equal-length sequences (one launch over strided views)
-    against the fixed-length entry points on contiguous [s, b, h, d] copies."""
+def test_varlen_api_with_equal_lengths_matches_the_fixed_length_entry_points():
+    """``pymha_varlen_fwd / bwd`` on a packed batch of equal-length sequences against the fixed-length entry points on contiguous
+    [s, b, h, d] copies."""
     from dhellam_b200.ops.attention import attn_bwd, attn_fwd, pymha_varlen_bwd, pymha_varlen_fwd
     b, s, hq, hk, d = 3, 256, 4, 2, 128
     cu = torch.arange(0, (b + 1) * s, s, dtype=torch.int32, device=DEV)
@@ -498,6 +507,9 @@ def test_packed_attention_against_fp32_sequence_by_sequence(ql, kl, causal, hq, 
     cpu = lambda t, c, i: t[c[i]:c[i + 1]].unsqueeze(1).float().cpu()
     got, want = [[] for _ in range(5)], [[] for _ in range(5)]
     for i in range(len(ql)):
+        assert (lse[i, :, ql[i]:] == float("-inf")).all()
+        if ql[i] == 0:                                     # keys that no query sees have no gradient
+            assert not dk[ck[i]:ck[i + 1]].any() and not dv[ck[i]:ck[i + 1]].any()
         if i == sick or ql[i] == 0:
             continue
         qi, ki, vi, di = cpu(q, cq, i), cpu(k, ck, i), cpu(v, ck, i), cpu(do, cq, i)
@@ -509,6 +521,54 @@ def test_packed_attention_against_fp32_sequence_by_sequence(ql, kl, causal, hq, 
             b.append(y.flatten())
     for name, a, b, tol in zip(("out", "lse", "dq", "dk", "dv"), got, want, (1e-2, 1e-3, 2e-2, 2e-2, 2e-2)):
         assert rel(torch.cat(a), torch.cat(b)) < tol, (name, rel(torch.cat(a), torch.cat(b)))
+
+
+@pytest.mark.parametrize("Sq,Sk", [(300, 40), (200, 130), (600, 129)])
+@pytest.mark.parametrize("packed", [False, True], ids=["dense", "packed"])
+def test_causal_queries_before_the_first_key(Sq, Sk, packed):
+    """More queries than keys, aligned at the end: the first Sq - Sk rows see no key (zeros, statistics of -inf, no gradient), in
+    whole tiles and in part of one; the others are the square problem of the last Sk rows."""
+    from dhellam_b200.ops.attention import attn_bwd, attn_fwd, pymha_varlen_bwd, pymha_varlen_fwd
+    q, k, v, do = bf(Sq, 1, 4, 128), bf(Sk, 1, 2, 128), bf(Sk, 1, 2, 128), bf(Sq, 1, 4, 128)
+    if packed:                                             # between two other sequences
+        sq, sk = [70, Sq, 131], [70, Sk, 131]
+        off = lambda n: [sum(n[:i]) for i in range(len(n) + 1)]
+        cq, ck, mid_q, mid_k = off(sq), off(sk), slice(70, 70 + Sq), slice(70, 70 + Sk)
+        around = lambda t: torch.cat([bf(70, *t.shape[2:]), t[:, 0], bf(131, *t.shape[2:])])
+        Q, K_, V, DO = around(q), around(k), around(v), around(do)
+        out, lse = pymha_varlen_fwd(Q, K_, V, cq, ck, max(sq), max(sk))
+        dq, dk, dv = pymha_varlen_bwd(DO, Q, K_, V, out, lse, cq, ck, max(sq), max(sk))
+        o, dq, dk, dv = (t[s].unsqueeze(1) for t, s in ((out, mid_q), (dq, mid_q), (dk, mid_k), (dv, mid_k)))
+        lse = lse[1:2, :, :Sq]
+    else:
+        o, lse = attn_fwd(q, k, v, True)
+        dq, dk, dv = attn_bwd(do, q, k, v, o, lse, True)
+    n = Sq - Sk
+    assert not o[:n].any() and not dq[:n].any() and (lse[:, :, :n] == float("-inf")).all()
+    qc, kc, vc, dc = (t.float().cpu() for t in (q[n:], k, v, do[n:]))
+    oref, lref = attn_fwd(qc, kc, vc, True)
+    grads = attn_bwd(dc, qc, kc, vc, oref, lref, True)
+    assert rel(o[n:], oref) < 1e-2 and rel(lse[:, :, n:], lref) < 1e-3
+    for a, b in zip((dq[n:], dk, dv), grads):
+        assert rel(a, b) < 2e-2
+
+
+def test_packed_batch_of_several_launches_equals_the_dense_kernels():
+    """More than 768 tiles and more than 128 sequences: cut into several launches, each tile as the dense kernels compute it."""
+    from dhellam_b200.ops.attention import attn_bwd, attn_fwd, pymha_varlen_bwd, pymha_varlen_fwd
+    lengths, hq, hk, d = [1000] * 100 + [130] * 60, 2, 1, 128
+    cu = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    q, k, v, do = bf(cu[-1], hq, d), bf(cu[-1], hk, d), bf(cu[-1], hk, d), bf(cu[-1], hq, d)
+    out, lse = pymha_varlen_fwd(q, k, v, cu, cu, 1000, 1000)
+    grads = pymha_varlen_bwd(do, q, k, v, out, lse, cu, cu, 1000, 1000)
+    for first, n, s in ((0, 100, 1000), (100, 60, 130)):
+        rows = slice(cu[first], cu[first + n])
+        sb = lambda t: t[rows].view(n, s, t.shape[1], d).permute(1, 0, 2, 3)
+        o, l = attn_fwd(sb(q), sb(k), sb(v), True)
+        assert torch.equal(sb(out), o) and torch.equal(lse[first:first + n, :, :s], l)
+        assert (lse[first:first + n, :, s:] == float("-inf")).all()
+        for a, b in zip(grads, attn_bwd(sb(do), sb(q), sb(k), sb(v), o, l, True)):
+            assert rel(sb(a), b) < 1e-3                    # the heads of a KV head may be divided otherwise: sums in another order
 
 
 def test_packed_attention_with_operands_of_different_lengths():
