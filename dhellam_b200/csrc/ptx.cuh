@@ -229,23 +229,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_bf16_2sm(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// A operand from TMEM (bf16 packed), B from shared memory.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // The same, issued by the lane whose `leader` is 1 while the WHOLE warp runs the instruction stream: without a
 // divergent branch around it the compiler keeps descriptors and addresses in uniform registers.  (Inside
 // `if (lane == 0)` every MMA first moved them there: 75-100 cycles each, more than a 128 x 128 MMA takes.)
@@ -258,6 +241,7 @@ __device__ __forceinline__ void umma_bf16_by(uint32_t leader, uint32_t tmem_d, u
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// A operand from TMEM (bf16 packed), B from shared memory.
 __device__ __forceinline__ void umma_bf16_ts_by(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                 uint32_t accumulate) {
   asm volatile(
@@ -278,6 +262,10 @@ __device__ __forceinline__ void umma_bf16_2sm_by(uint32_t leader, uint32_t tmem_
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// 2-SM commit: arrives on ONE barrier, named by a shared::cluster address, once all
+// MMAs issued so far by this thread for the CTA pair have retired.  To release a
+// stage in both CTAs of the pair issue it twice (own address, then the peer's
+// address obtained with mapa).
 __device__ __forceinline__ void umma_commit_2sm_by(uint32_t leader, uint32_t cluster_bar_addr) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -295,13 +283,6 @@ __device__ __forceinline__ void umma_commit_by(uint32_t leader, uint64_t* bar) {
 // Make the barrier complete once all previously issued MMAs of this thread retire.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// 2-SM commit: arrives on ONE barrier, named by a shared::cluster address, once all
-// MMAs issued so far by this thread for the CTA pair have retired.  To release a
-// stage in both CTAs of the pair issue it twice (own address, then the peer's
-// address obtained with mapa).
-__device__ __forceinline__ void umma_commit_2sm(uint32_t cluster_bar_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar_addr) : "memory");
 }
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t cta) {
   uint32_t remote;
