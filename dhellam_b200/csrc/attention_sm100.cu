@@ -13,13 +13,16 @@
 //   warp 1      MMA issuer:   S_t = Q_t K_j^T, O_t += P_t V_j (t = 0, 1) with P read from TMEM
 //   warps 4-7, 8-11  softmax of tile 0 / 1: one thread per row, no exchange between threads; P_t
 //               overwrites S_t in TMEM as bf16; O_t stays in TMEM and is rescaled when the maximum
-//               of one of the warp's rows has grown.  (Keeping a maximum until it has grown by a
-//               factor, as published for flash attention on this hardware, is faster but less exact:
-//               the largest probability of a row is then rounded to bf16 where it would be exactly 1.)
+//               of one of the warp's rows has grown.  (Two tiles with P over S in TMEM and a rescaling
+//               only when the maximum has grown by a factor are the scheme published as
+//               FlashAttention-4.  The factor is left out: with it the largest probability of a row
+//               is rounded to bf16 where it would be exactly 1.  Error of the output against 64
+//               bits, factor 2^8 and without: 0.00201 and 0.00198 for scores of standard deviation
+//               1, 0.00207 and 0.00177 for 3; 432 and 473 us on 16384 positions.)
 //   While one tile is in softmax the tensor cores work on the other.
-//   Measured, causal, 8 query heads on 2 KV heads: 32768 positions inside a training step (power-capped clocks) 3628 -> 2099 us,
-//   16384 positions alone 452 us (1.22 PFLOP/s);
-//   tensor and special-function pipes each ~66 % busy, the rest is the chain softmax -> P V -> S of one tile (two softmax
+//   Measured, causal, 8 query heads on 2 KV heads: 32768 positions inside a training step (power-capped clocks) 3628 -> 2098 us,
+//   16384 positions alone 866 -> 478 us (1.15 PFLOP/s);
+//   tensor and special-function pipes each ~55 % busy, the rest is the chain softmax -> P V -> S of one tile (two softmax
 //   warps per scheduler).  Tried and slower: steps of 64 keys with S double-buffered (an N = 64 product takes as long as an
 //   N = 128 one: 2116 against 1550 cycles per tile pair); 1/8 to 1/2 of the exponentials as a polynomial on the FMA pipe
 //   (4 to 20 % slower: the warps are bound by instruction latency, not by the special-function pipe).
@@ -32,13 +35,13 @@
 //     read half the shared memory.  The math warps' P phase runs beside dK(i-1), dP(i) and the dS
 //     phase beside dV(i), S(i+1), so nothing is double-buffered in TMEM.  When keys x batch x KV
 //     heads gives too few CTAs (one KV head per GPU under tensor parallelism), the query heads
-//     of a group are split over up to 8 CTAs that write fp32 partials; attn_dkv_reduce_kernel
-//     adds them in a fixed order.
+//     of a group are split over a power of two of CTAs that write fp32 partials (bwd_head_split);
+//     attn_dkv_reduce_kernel adds them in a fixed order.
 //   dQ: one CTA per (128 queries, batch, query head) loops over the key blocks, recomputes S
 //     and dP and accumulates dQ += dS K in TMEM (dS again as a TMEM operand).  Recomputing two
 //     products per tile pair replaces an fp32 atomic accumulation of dQ and keeps dQ reproducible.
-//   Measured (32768 positions in the step): dK/dV 7833 -> 4071 us, dQ 5326 -> 2708 us; 16384 alone 867 and 568 us.  The forms before ran one phase after
-//   the other and applied the mask as predicates (10 ALU instructions per score in dQ).
+//   Measured (32768 positions in the step): dK/dV 7833 -> 3844 us, dQ 5326 -> 2630 us; 16384 alone, both and delta 2856 -> 1455 us.  The forms before
+//   ran one phase after the other and applied the mask as predicates (10 ALU instructions per score in dQ).
 //
 // MMAs are issued under a predicate by a warp whose control flow stays uniform (ptx.cuh, umma_bf16_by): issued inside
 // `if (lane == 0)` a 128 x 128 x 16 product took 75-100 cycles to issue, against 64 to execute.

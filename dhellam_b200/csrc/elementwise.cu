@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(NT) norm_bwd_kernel(const __nv_bfloat16* __res
 // vectors.  The kernel is bound by memory; the form above keeps a row's loads behind the previous row's reduction, with 170
 // registers and one CTA of 8 warps per SM (two at 4096), and loads the residual after the reduction.  Here the registers
 // do not grow with the row and the next row's three loads are in flight while this row is reduced (one barrier per row).
-//   4096 x 4096 56 -> 40 us, 32768 x 4096 371 -> 228 us (4.7 TB/s), 4096 x 8192 173 -> 82 us, layer norm 3800 x 5120 123 -> 65 us.
+//   Cold L2: 4096 x 4096 55 -> 35 us, 32768 x 4096 356 -> 186 us (5.8 TB/s), 4096 x 8192 157 -> 64 us, layer norm 3800 x 5120 82 -> 51 us.
 // The forward keeps several vectors per thread: its rows are independent CTAs and it was faster so (4096 x 8192 33 against 54 us).
 constexpr int ROW_MAXT = 1024;
 static inline int row_threads(int h) { return ((h >> 3) + 31) & ~31; }

@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(256) moe_dispatch_kernel(const DispatchParams 
     const uint4* oth = p.other != nullptr ? reinterpret_cast<const uint4*>(p.other + (long long)i * p.h) : nullptr;
     float dot = 0.f;
     // A warp moves a row in pieces of VPL vectors per lane, all loads of a piece in flight before the first is used: a row
-    // is a dependent chain otherwise.  8192 rows of 8 KB on one GPU: 141 us -> 27 us (with the grid of exchange_ctas), combine 177 -> 24 us.
+    // is a dependent chain otherwise.  8192 rows of 8 KB on one GPU, cold L2: 139 us -> 25 us (with the grid of exchange_ctas), combine
+    // 164 -> 21 us.
     for (int v0 = lane; v0 < vecs; v0 += 32 * VPL) {
       uint4 xs[VPL], ys[VPL];
 #pragma unroll

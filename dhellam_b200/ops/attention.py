@@ -179,7 +179,7 @@ def _as_sbhd(t, b, s):
 
 
 def _runs_packed(q, k, cq, ck, max_q) -> bool:
-    """Whether a packed batch runs as ONE launch of the packed kernels (offsets as kernel parameters, tiles of all
+    """Whether a packed batch runs on the packed kernels (offsets as kernel parameters, tiles of all
     sequences in descending order of work): CUDA tensors with offsets that ascend and stay inside the tensors and
     within ``max_q``.  Everything else (CPU, library backend, offsets that do not describe the tensors) takes the
     sequence-by-sequence path, which also reports what is wrong with them."""
@@ -200,8 +200,8 @@ def pymha_varlen_fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
     """Packed variable-length attention with the reference's signature
     (csrc/operators/ops.h:18-32): ``q [total_q, h, d]``, ``k, v [total_k, h_k, d]`` and
     cumulative sequence offsets.  Returns ``(out [total_q, h, d], softmax_lse [b, h, max_q])``.
-    The whole batch is one launch, whatever the lengths.  Attention dropout is not supported by the sm_100a kernel
-    (``p_dropout`` must be 0)."""
+    The whole batch is one launch, whatever the lengths, up to 128 sequences and 768 tiles of 128 rows; larger ones are cut
+    into a few.  Attention dropout is not supported by the sm_100a kernel (``p_dropout`` must be 0)."""
     assert p_dropout == 0.0, "attention dropout is not implemented"
     cq, ck = _offset_pair(cu_seqlens_q, cu_seqlens_k)
     b = len(cq) - 1
