@@ -1285,11 +1285,12 @@ static int gemm_impl(const void* a, int64_t lda, int a_mn_major, const void* b, 
 extern "C" void dh_gemm_set_splitk(int n) { dh::gemm::g_splitk_override = n; }
 
 // Small-output kernel (128 x 128 tiles, K over a cluster): -1 = by problem (default), 0 = never, n = n CTAs per tile.
-// That rule (or the forced number) for a problem on `sms` SMs.
+extern "C" void dh_gemm_set_cluster_k(int n) { dh::gemm::g_cluster_k = n; }
+
+// What that comes to for a problem on `sms` SMs.
 extern "C" int dh_gemm_cluster_k(int M, int N, int K, int out_f32, int sms) {
   return dh::gemm::choose_cluster_k(M, N, (K + dh::gemm::BK - 1) / dh::gemm::BK, out_f32, sms);
 }
-extern "C" void dh_gemm_set_cluster_k(int n) { dh::gemm::g_cluster_k = n; }
 
 extern "C" int dh_gemm_bf16(const void* a, int64_t lda, int a_mn_major, const void* b, int64_t ldb, int b_mn_major, void* d,
                             int64_t ldd, int d_fp32, int accumulate, int M, int N, int K, int epilogue, int sm_budget,
